@@ -30,7 +30,7 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-Xcompiler", "-fPIC", "-shared",
-    "--expt-relaxed-constexpr",
+    "--expt-relaxed-constexpr", "-split-compile=0",
     "-Xcompiler", "-fopenmp", "-lgomp",
 ]
 

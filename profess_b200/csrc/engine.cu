@@ -954,13 +954,11 @@ struct Engine {
       }
 #else
     double* dq = nullptr;
-    if ((rc = dmalloc((void**)&dq, sizeof(double) * q.size()))) return rc;
+    if ((rc = io_scratch(sizeof(double) * q.size(), (void**)&dq))) return rc;
     if (h.prec == OFDFT_FP32) k_force_gather<float><<<h.nion, 256, 0, stream>>>(d_slots + i, h.d_stencil, dq);
     else k_force_gather<double><<<h.nion, 256, 0, stream>>>(d_slots + i, h.d_stencil, dq);
     rc = cuda_check(cudaGetLastError(), "force gather launch");
-    if (!rc) rc = sync_stream();
     if (!rc) rc = d2h(q.data(), dq, sizeof(double) * q.size());
-    dfree(dq);
     if (rc) return rc;
 #endif
     // F_ie = -cellInv * sum(qIonDeriv * Factor) (CalculateSplineForces)
@@ -1042,7 +1040,7 @@ struct Engine {
     sa.kf = std::cbrt(3.0 * PI_D * PI_D * (wgc ? s.rho_s : h.rho0));
     sa.ki = 20.0 * std::pow(h.rho0, 5.0 / 3.0 - (s.alpha + s.beta));
     sa.gamma = h.gamma;
-    const int nblk = (int)std::max<long long>(1, std::min<long long>(2 * (long long)num_sms, (s.Nc + 127) / 128));
+    const int nblk = std::min(6 * num_sms, s.k1 * s.n2);  // rows (kx, y) spread over them
     std::vector<double> part((size_t)NSC * nblk);
 #if defined(OFDFT_EMU)
     std::vector<cx<double>> sf((size_t)nion * L);
@@ -1053,15 +1051,16 @@ struct Engine {
     sa.sf = sf.data();
     sa.species = species.data();
     double red[NSC];
+    std::vector<cx<double>> prod(STRESS_CHUNK);
     for (int b = 0; b < nblk; ++b) {
-      if (h.prec == OFDFT_FP32) stress_block<float>(s, sa, b, nblk, 0, 1, red, &part[(size_t)NSC * b]);
-      else stress_block<double>(s, sa, b, nblk, 0, 1, red, &part[(size_t)NSC * b]);
+      if (h.prec == OFDFT_FP32) stress_block<float>(s, sa, b, nblk, 0, 1, prod.data(), red, &part[(size_t)NSC * b]);
+      else stress_block<double>(s, sa, b, nblk, 0, 1, prod.data(), red, &part[(size_t)NSC * b]);
     }
 #else
     const size_t sf_bytes = sizeof(cx<double>) * (size_t)nion * L;
     const size_t part_bytes = sizeof(double) * part.size();
     char* scratch = nullptr;
-    if ((rc = dmalloc((void**)&scratch, sf_bytes + part_bytes + sizeof(int) * (size_t)nion))) return rc;
+    if ((rc = io_scratch(sf_bytes + part_bytes + sizeof(int) * (size_t)nion, (void**)&scratch))) return rc;
     cx<double>* dsf = (cx<double>*)scratch;
     double* dpart = (double*)(scratch + sf_bytes);
     int* dspec = (int*)(scratch + sf_bytes + part_bytes);
@@ -1077,7 +1076,6 @@ struct Engine {
       rc = cuda_check(cudaGetLastError(), "stress launch");
     }
     if (!rc) rc = d2h(part.data(), dpart, part_bytes);
-    dfree(scratch);
     if (rc) return rc;
 #endif
     double acc[NSC] = {0};
@@ -1136,12 +1134,11 @@ struct Engine {
     }
 #else
     double* dp = nullptr;
-    if ((rc = dmalloc((void**)&dp, sizeof(double) * nblk))) return rc;
+    if ((rc = io_scratch(sizeof(double) * nblk, (void**)&dp))) return rc;
     if (h.prec == OFDFT_FP32) k_sum<float><<<nblk, 256, 0, stream>>>((const float*)h.input, s.N, dp);
     else k_sum<double><<<nblk, 256, 0, stream>>>((const double*)h.input, s.N, dp);
     rc = cuda_check(cudaGetLastError(), "sum launch");
     if (!rc) rc = d2h(part.data(), dp, sizeof(double) * nblk);
-    dfree(dp);
     if (rc) return rc;
 #endif
     double sum = 0.0;
@@ -1178,13 +1175,12 @@ struct Engine {
     }
 #else
     double* dp = nullptr;
-    int rc = dmalloc((void**)&dp, sizeof(double) * nblk);
+    int rc = io_scratch(sizeof(double) * nblk, (void**)&dp);
     if (rc) return rc;
     if (h.prec == OFDFT_FP32) k_rho_vxc<float><<<nblk, 256, 0, stream>>>((const float*)s.buf[b], s.N, dp);
     else k_rho_vxc<double><<<nblk, 256, 0, stream>>>((const double*)s.buf[b], s.N, dp);
     rc = cuda_check(cudaGetLastError(), "rho vxc launch");
     if (!rc) rc = d2h(part.data(), dp, sizeof(double) * nblk);
-    dfree(dp);
     if (rc) return rc;
 #endif
     double sum = 0.0;
@@ -1198,45 +1194,19 @@ struct Engine {
     HostSlot& h = slots[i];
     const int nion = h.nion;
     const EwaldPar p = ewald_par(h.lattice, nion);
-    const int npl = ewald_planes(p);
-    std::vector<double> pos(3 * (size_t)nion);
-    for (int k = 0; k < nion; ++k)
-      for (int r = 0; r < 3; ++r)
-        pos[3 * k + r] = p.A[r][0] * h.frac[3 * k] + p.A[r][1] * h.frac[3 * k + 1] + p.A[r][2] * h.frac[3 * k + 2];
-    std::vector<double> real7(7 * (size_t)nion), plane7(7 * (size_t)npl);
-#if defined(OFDFT_EMU)
-    double red[7];
-    for (int k = 0; k < nion; ++k) ewald_real_stress_block(p, pos.data(), h.zion.data(), k, 0, 1, red, &real7[7 * k]);
-    for (int m = 0; m < npl; ++m)
-      ewald_plane_stress_block(p, h.frac.data(), h.zion.data(), m, 0, 1, red, &plane7[7 * m]);
-#else
-    const size_t nd = 3 * (size_t)nion * 2 + nion + 7 * (size_t)nion + 7 * (size_t)npl;
-    double* dbuf = nullptr;
-    int rc = dmalloc((void**)&dbuf, sizeof(double) * nd);
+    const int rows = ewald_rows(p);
+    std::vector<double> out;
+    const int rc = ewald_sums<7>(h, p, false, out);
     if (rc) return rc;
-    double *dpos = dbuf, *dfrac = dpos + 3 * nion, *dz = dfrac + 3 * nion, *dreal = dz + nion, *dplane = dreal + 7 * nion;
-    rc = h2d(dpos, pos.data(), sizeof(double) * 3 * nion);
-    if (!rc) rc = h2d(dfrac, h.frac.data(), sizeof(double) * 3 * nion);
-    if (!rc) rc = h2d(dz, h.zion.data(), sizeof(double) * nion);
-    if (!rc) {
-      k_ewald_real_stress<<<nion, 128, 0, stream>>>(p, dpos, dz, dreal);
-      k_ewald_plane_stress<<<npl, 128, 0, stream>>>(p, dfrac, dz, dplane);
-      rc = cuda_check(cudaGetLastError(), "Ewald stress launch");
-    }
-    if (!rc) rc = d2h(real7.data(), dreal, sizeof(double) * 7 * nion);
-    if (!rc) rc = d2h(plane7.data(), dplane, sizeof(double) * 7 * npl);
-    dfree(dbuf);
-    if (rc) return rc;
-#endif
     double qsum = 0.0, e_rec = 0.0, s6[6] = {0};
     for (int k = 0; k < nion; ++k) {
       qsum += h.zion[k];
-      for (int c = 0; c < 6; ++c) s6[c] += real7[7 * k + 1 + c];
+      for (int c = 0; c < 6; ++c) s6[c] += out[7 * (size_t)k + 1 + c];
     }
     double r6[6] = {0};
-    for (int m = 0; m < npl; ++m) {
-      e_rec += plane7[7 * m];
-      for (int c = 0; c < 6; ++c) r6[c] += plane7[7 * m + 1 + c];
+    for (int r = 0; r < rows; ++r) {
+      e_rec += out[7 * (size_t)(nion + r)];
+      for (int c = 0; c < 6; ++c) r6[c] += out[7 * (size_t)(nion + r) + 1 + c];
     }
     const double e_bg = -0.5 * PI_D / (p.eta * p.eta) / p.vol * qsum * qsum;
     for (int c = 0; c < 6; ++c) {
@@ -1281,7 +1251,16 @@ struct Engine {
       d_io = nullptr;
       io_bytes = 0;
       int rc = cuda_check(cudaMalloc(&d_io, bytes), "cudaMalloc");
-      if (rc) return rc;
+      if (rc == OFDFT_ENOMEM) {
+        cudaGetLastError();  // must not show up as a later launch error
+        pool_flush();
+        rc = cuda_check(cudaMalloc(&d_io, bytes), "cudaMalloc");
+      }
+      if (rc) {
+        cudaGetLastError();
+        d_io = nullptr;
+        return rc;
+      }
       io_bytes = bytes;
     }
     *p = d_io;
@@ -1416,64 +1395,79 @@ struct Engine {
     return OFDFT_OK;
   }
 
+  // Device sums of the Ewald series of slot h's ions (ewald.cuh).  out gets
+  // NOUT values per ion (real space) and per reciprocal row, then, with force,
+  // three values per ion (reciprocal forces).
+  template <int NOUT>
+  int ewald_sums(const HostSlot& h, const EwaldPar& p, bool force, std::vector<double>& out) {
+    const int nion = h.nion, rows = ewald_rows(p), nsum = nion + rows, nph = ewald_phases(p);
+    const size_t nsf = (size_t)rows * ewald_nm(p, 2);
+    out.resize((size_t)NOUT * nsum + (force ? 3 * (size_t)nion : 0));
+    double* orec = out.data() + (size_t)NOUT * nsum;
+#if defined(OFDFT_EMU)
+    std::vector<cx<double>> tab(nph), sf(nsf), prod(EWALD_CHUNK), part(EWALD_M3);
+    double red[NOUT];
+    const double *frac = h.frac.data(), *z = h.zion.data();
+    for (int w = 0; w < nph; ++w) tab[w] = ewald_phase(p, frac, w);
+    for (int k = 0; k < nion; ++k) {
+      if constexpr (NOUT == 7) ewald_real_stress_block(p, frac, z, k, 0, 1, red, &out[(size_t)NOUT * k]);
+      else ewald_real_block(p, frac, z, k, 0, 1, red, &out[(size_t)NOUT * k]);
+    }
+    for (int r = 0; r < rows; ++r)
+      ewald_row_block<NOUT == 7 ? 7 : 1>(p, tab.data(), z, r, 0, 1, prod.data(), part.data(), red, sf.data(),
+                                         &out[(size_t)NOUT * (nion + r)]);
+    if (force)
+      for (int k = 0; k < nion; ++k)
+        ewald_recip_force_block(p, tab.data(), z, sf.data(), k, 0, 1, red, orec + 3 * (size_t)k);
+    return OFDFT_OK;
+#else
+    // one scratch array (the engine's transfer scratch): phases, S(G), the
+    // outputs, then frac and z (one copy up, one copy down)
+    std::vector<double> in(h.frac);
+    in.insert(in.end(), h.zion.begin(), h.zion.end());
+    char* scratch = nullptr;
+    int rc = io_scratch(sizeof(cx<double>) * (nph + nsf) + sizeof(double) * (out.size() + in.size()), (void**)&scratch);
+    if (rc) return rc;
+    cx<double>* dtab = (cx<double>*)scratch;
+    cx<double>* dsf = dtab + nph;
+    double* dout = (double*)(dsf + nsf);
+    double* dfrac = dout + out.size();
+    double* dz = dfrac + 3 * (size_t)nion;
+    if ((rc = h2d(dfrac, in.data(), sizeof(double) * in.size()))) return rc;
+    k_ewald_phase<<<(nph + 255) / 256, 256, 0, stream>>>(p, dfrac, dtab);
+    k_ewald_sums<NOUT><<<nsum, 128, 0, stream>>>(p, dfrac, dz, dtab, dsf, dout);
+    if (force) k_ewald_recip_force<<<nion, 128, 0, stream>>>(p, dtab, dz, dsf, dout + (orec - out.data()));
+    if ((rc = cuda_check(cudaGetLastError(), "Ewald launch"))) return rc;
+    return d2h(out.data(), dout, sizeof(double) * out.size());
+#endif
+  }
+
   // Ewald energy and forces (Ha, Ha/bohr; forces may be NULL) of the slot's
   // ions, summed on the device.
   int ewald_device(int i, double* energy, double* forces) {
-    int rc = OFDFT_OK;
     HostSlot& h = slots[i];
     const int nion = h.nion;
     if (nion < 1) return fail(OFDFT_EINVAL, "build the ion potential before the Ewald sum");
     const EwaldPar p = ewald_par(h.lattice, nion);
-    const int npl = ewald_planes(p), plane = ewald_plane_size(p);
-    std::vector<double> pos(3 * (size_t)nion);
-    for (int k = 0; k < nion; ++k)
-      for (int r = 0; r < 3; ++r)
-        pos[3 * k + r] = p.A[r][0] * h.frac[3 * k] + p.A[r][1] * h.frac[3 * k + 1] + p.A[r][2] * h.frac[3 * k + 2];
-    std::vector<double> real4(4 * (size_t)nion), plane4(4 * (size_t)npl), rec4(4 * (size_t)nion);
-#if defined(OFDFT_EMU)
-    std::vector<cx<double>> sfac((size_t)npl * plane);
-    double red[4];
-    for (int k = 0; k < nion; ++k) ewald_real_block(p, pos.data(), h.zion.data(), k, 0, 1, red, &real4[4 * k]);
-    for (int m = 0; m < npl; ++m) ewald_plane_block(p, h.frac.data(), h.zion.data(), m, 0, 1, red, sfac.data(), &plane4[4 * m]);
-    if (forces)
-      for (int k = 0; k < nion; ++k)
-        ewald_recip_force_block(p, h.frac.data(), h.zion.data(), sfac.data(), k, 0, 1, red, &rec4[4 * k]);
-#else
-    // one scratch array (the engine's transfer scratch): pos, frac, z, the three
-    // 4-value outputs, S(G)
-    const size_t nd = 3 * (size_t)nion * 2 + nion + 4 * (size_t)nion * 2 + 4 * (size_t)npl;
-    double* dbuf = nullptr;
-    if ((rc = io_scratch(sizeof(double) * nd + sizeof(cx<double>) * (size_t)npl * plane, (void**)&dbuf))) return rc;
-    double *dpos = dbuf, *dfrac = dpos + 3 * nion, *dz = dfrac + 3 * nion, *dreal = dz + nion, *drec = dreal + 4 * nion,
-           *dplane = drec + 4 * nion;
-    cx<double>* dsf = (cx<double>*)(dbuf + nd);
-    rc = h2d(dpos, pos.data(), sizeof(double) * 3 * nion);
-    if (!rc) rc = h2d(dfrac, h.frac.data(), sizeof(double) * 3 * nion);
-    if (!rc) rc = h2d(dz, h.zion.data(), sizeof(double) * nion);
-    if (!rc) {
-      k_ewald_real<<<nion, 256, 0, stream>>>(p, dpos, dz, dreal);
-      k_ewald_plane<<<npl, 256, 0, stream>>>(p, dfrac, dz, dsf, dplane);
-      if (forces) k_ewald_recip_force<<<nion, 256, 0, stream>>>(p, dfrac, dz, dsf, drec);
-      rc = cuda_check(cudaGetLastError(), "Ewald launch");
-    }
-    if (!rc) rc = d2h(real4.data(), dreal, sizeof(double) * 4 * nion);
-    if (!rc) rc = d2h(plane4.data(), dplane, sizeof(double) * 4 * npl);
-    if (!rc && forces) rc = d2h(rec4.data(), drec, sizeof(double) * 4 * nion);
+    const int rows = ewald_rows(p);
+    std::vector<double> out;
+    const int rc = ewald_sums<4>(h, p, forces != nullptr, out);
     if (rc) return rc;
-#endif
     double qsum = 0.0, q2 = 0.0, e_real = 0.0, e_rec = 0.0;
     for (int k = 0; k < nion; ++k) {
       qsum += h.zion[k];
       q2 += h.zion[k] * h.zion[k];
-      e_real += real4[4 * k];
+      e_real += out[4 * (size_t)k];
     }
-    for (int m = 0; m < npl; ++m) e_rec += plane4[4 * m];
+    for (int r = 0; r < rows; ++r) e_rec += out[4 * (size_t)(nion + r)];
     const double e_self = -p.eta / std::sqrt(PI_D) * q2;
     const double e_bg = -0.5 * PI_D / (p.eta * p.eta) / p.vol * qsum * qsum;
     const double e = e_real + e_self + e_rec + e_bg;
-    if (forces)
+    if (forces) {
+      const double* rec = out.data() + 4 * (size_t)(nion + rows);
       for (int k = 0; k < nion; ++k)
-        for (int r = 0; r < 3; ++r) forces[3 * k + r] = real4[4 * k + 1 + r] + rec4[4 * k + 1 + r];
+        for (int r = 0; r < 3; ++r) forces[3 * k + r] = out[4 * (size_t)k + 1 + r] + rec[3 * (size_t)k + r];
+    }
     if (energy) *energy = e;
     return OFDFT_OK;
   }
@@ -2080,8 +2074,8 @@ struct Engine {
     cudaFuncAttributes fa;
     int rc = preload_prec<float>();
     if (!rc) rc = preload_prec<double>();
-    for (const void* k : {(const void*)k_ewald_real, (const void*)k_ewald_plane, (const void*)k_ewald_recip_force,
-                          (const void*)k_ewald_real_stress, (const void*)k_ewald_plane_stress, (const void*)k_stress_sf})
+    for (const void* k : {(const void*)k_ewald_phase, (const void*)k_ewald_sums<4>, (const void*)k_ewald_sums<7>,
+                          (const void*)k_ewald_recip_force, (const void*)k_stress_sf})
       if (!rc) rc = cuda_check(cudaFuncGetAttributes(&fa, k), "kernel load");
     return rc;
   }

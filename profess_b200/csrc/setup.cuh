@@ -375,6 +375,7 @@ struct EwaldPar {
   double inv[3][3];  // inverse of A
   double vol, eta, rcut, gcut;
   int nimg[3], ng[3];
+  int nw[3];  // image range of a difference wrapped to [-1/2, 1/2] (device sum)
   int nion;
 };
 
@@ -405,6 +406,7 @@ inline EwaldPar ewald_par(const double* L, int nion) {
   for (int a = 0; a < 3; ++a) {
     const double hr = 1.0 / std::sqrt(inv[a][0] * inv[a][0] + inv[a][1] * inv[a][1] + inv[a][2] * inv[a][2]);
     p.nimg[a] = (int)std::ceil(p.rcut / hr) + 1;
+    p.nw[a] = (int)std::floor(p.rcut / hr + 0.5 + 1e-9);
     // reciprocal vector a has length 2 pi |row a of inv|; plane spacing in G space
     double la = 0;
     for (int k = 0; k < 3; ++k) la += A[k][a] * A[k][a];

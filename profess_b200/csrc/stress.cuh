@@ -133,15 +133,6 @@ HD cx<double> stress_sf_entry(const SlotDev& s, const IonStencil& st, int w) {
   return mk<double>(re, im);
 }
 
-HD void sym_add(double* a, const double* g, double w) {
-  a[0] += w * g[0] * g[0];
-  a[1] += w * g[0] * g[1];
-  a[2] += w * g[0] * g[2];
-  a[3] += w * g[1] * g[1];
-  a[4] += w * g[1] * g[2];
-  a[5] += w * g[2] * g[2];
-}
-
 template <typename T>
 HD cx<double> spec_at(const SlotDev& s, int f, long long p) {
   const cx<T> v = ((const cx<T>*)s.spec)[(size_t)f * (size_t)s.Nc + (size_t)p];
@@ -193,13 +184,13 @@ HD void stress_wgc_point(const SlotDev& s, const StressArgs& sa, long long p, co
   sym_add(acc + SC_WT, g, offdia / q2);
 }
 
-// The terms of stored frequency p (kx-major position) added to acc[NSC].
+// The terms of stored frequency p = (kx, position yi, position zi), whose
+// natural indices are (kx, ky, kz), added to acc[NSC].  st[sp] is species
+// sp's structure factor there, without the B-spline factor b1 b2 b3.
 template <typename T>
-HD void stress_point(const SlotDev& s, const StressArgs& sa, long long p, double* acc) {
-  const int n1 = s.n1, n2 = s.n2, n3 = s.n3, nrows = n2 * n3;
-  const int kx = (int)(p / nrows), j = (int)(p - (long long)kx * nrows);
-  const int zi = j / n2, yi = j - zi * n2;
-  const int ky = sa.permy[yi], kz = sa.permz[zi];
+HD void stress_point(const SlotDev& s, const StressArgs& sa, long long p, int kx, int ky, int kz,
+                     const cx<double>* st, double* acc) {
+  const int n1 = s.n1, n2 = s.n2, n3 = s.n3;
   const int m2 = signed_freq(ky, n2), m3 = signed_freq(kz, n3);
   const double* R = s.recip;
   double g[3], ge[3];
@@ -234,16 +225,13 @@ HD void stress_point(const SlotDev& s, const StressArgs& sa, long long p, double
   }
   // ion-electron
   if (sa.nion > 0) {
-    double vp[MAX_SPECIES];
-    for (int sp = 0; sp < s.ion.nspec; ++sp) vp[sp] = psp_diff(s.ion, sp, q) / q;
-    const int L = s.k1 + n2 + n3;
     double tr = 0.0, ti = 0.0;
-    for (int i = 0; i < sa.nion; ++i) {
-      const cx<double>* A = sa.sf + (size_t)i * L;
-      const cx<double> a = cmul(cmul(A[kx], A[s.k1 + ky]), A[s.k1 + n2 + kz]);
-      const double v = vp[sa.species[i]];
-      tr += a.x * v;
-      ti += a.y * v;
+#pragma unroll
+    for (int sp = 0; sp < MAX_SPECIES; ++sp) {
+      if (sp >= s.ion.nspec) break;
+      const double v = psp_diff(s.ion, sp, q) / q;
+      tr += st[sp].x * v;
+      ti += st[sp].y * v;
     }
     const cx<double> bb = cmul(cmul(s.ion.b1[kx], s.ion.b2[ky]), s.ion.b3[kz]);
     const cx<double> sf = cmul(bb, mk<double>(tr * s.inv_n, ti * s.inv_n));
@@ -251,29 +239,59 @@ HD void stress_point(const SlotDev& s, const StressArgs& sa, long long p, double
   }
 }
 
-// Fixed-order sum of K values per thread over the block; thread 0 writes
-// out[0..K-1].  red holds K * nthr doubles.
-template <int K>
-HD void block_sum(double* red, const double* v, int tid, int nthr, double* out) {
-  for (int k = 0; k < K; ++k) red[K * tid + k] = v[k];
-  BLOCK_SYNC();
-  for (int st = 1; st < nthr; st *= 2) {
-    if ((tid % (2 * st)) == 0 && tid + st < nthr)
-      for (int k = 0; k < K; ++k) red[K * tid + k] += red[K * (tid + st) + k];
-    BLOCK_SYNC();
-  }
-  if (tid == 0)
-    for (int k = 0; k < K; ++k) out[k] = red[k];
-}
-
-// Block b of nblk: frequencies p = b*nthr + tid + r*nblk*nthr.
+// Block b of nblk: the rows (kx, yi) r = b, b + nblk, ..., their zi spread over
+// the threads.  The structure factor of a row is a contraction over the ions,
+// sum_i (A_x A_y)_i A_z(i, kz): the products A_x A_y of a row go to shared
+// memory once (chunks of STRESS_CHUNK ions), so a frequency costs four
+// multiply-adds an ion instead of two complex products and the table loads
+// (108 ions, 72^3: see k_stress).
+constexpr int STRESS_CHUNK = 256;
 template <typename T>
-HD void stress_block(const SlotDev& s, const StressArgs& sa, int b, int nblk, int tid, int nthr, double* red,
-                     double* out) {
+HD void stress_block(const SlotDev& s, const StressArgs& sa, int b, int nblk, int tid, int nthr, cx<double>* prod,
+                     double* red, double* out) {
+  const int n2 = s.n2, n3 = s.n3, rows = s.k1 * n2, L = s.k1 + n2 + n3;
   double acc[NSC];
   for (int k = 0; k < NSC; ++k) acc[k] = 0.0;
-  const long long stride = (long long)nblk * nthr;
-  for (long long p = (long long)b * nthr + tid; p < s.Nc; p += stride) stress_point<T>(s, sa, p, acc);
+  for (int r = b; r < rows; r += nblk) {
+    const int kx = r / n2, yi = r - kx * n2, ky = sa.permy[yi];
+    for (int z0 = 0; z0 < n3; z0 += nthr) {
+      const int zi = z0 + tid, kz = zi < n3 ? sa.permz[zi] : 0;
+      cx<double> st[MAX_SPECIES];
+#pragma unroll
+      for (int sp = 0; sp < MAX_SPECIES; ++sp) st[sp] = mk<double>(0.0, 0.0);
+      for (int i0 = 0; i0 < sa.nion; i0 += STRESS_CHUNK) {
+        const int ni = sa.nion - i0 < STRESS_CHUNK ? sa.nion - i0 : STRESS_CHUNK;
+        BLOCK_SYNC();
+        for (int i = tid; i < ni; i += nthr) {
+          const cx<double>* A = sa.sf + (size_t)(i0 + i) * L;
+          prod[i] = cmul(A[kx], A[s.k1 + ky]);
+        }
+        BLOCK_SYNC();
+        const cx<double>* az = sa.sf + (size_t)i0 * L + s.k1 + n2 + kz;
+#pragma unroll
+        for (int sp = 0; sp < MAX_SPECIES; ++sp) {
+          if (sp >= s.ion.nspec) break;
+          if (s.ion.nspec == 1) {
+#pragma unroll 8
+            for (int i = 0; i < ni; ++i) {
+              const cx<double> x = cmul(prod[i], az[(size_t)i * L]);
+              st[sp].x += x.x;
+              st[sp].y += x.y;
+            }
+            break;
+          }
+          for (int i = 0; i < ni; ++i) {
+            if (sa.species[i0 + i] != sp) continue;
+            const cx<double> x = cmul(prod[i], az[(size_t)i * L]);
+            st[sp].x += x.x;
+            st[sp].y += x.y;
+          }
+        }
+      }
+      if (zi < n3) stress_point<T>(s, sa, ((long long)kx * n3 + zi) * n2 + yi, kx, ky, kz, st, acc);
+    }
+  }
+  BLOCK_SYNC();
   block_sum<NSC>(red, acc, tid, nthr, out);
 }
 
@@ -302,64 +320,6 @@ HD void sum_block(const T* v, long long n, int b, int nblk, int tid, int nthr, d
   block_sum<1>(red, &acc, tid, nthr, out);
 }
 
-// ---------------------------------------------------------------- Ewald stress
-// out7 = (0, the six components of sum 0.5 z_i z_j f'(r)/r d_a d_b) over the
-// images and partners of ion i, f(r) = erfc(eta r)/r.
-HD void ewald_real_stress_block(const EwaldPar& p, const double* pos, const double* z, int i, int tid, int nthr,
-                                double* red, double* out7) {
-  const int na = 2 * p.nimg[0] + 1, nb = 2 * p.nimg[1] + 1, nc = 2 * p.nimg[2] + 1;
-  const long long total = (long long)na * nb * nc * p.nion;
-  const double rc2 = p.rcut * p.rcut, eta = p.eta;
-  const double c2 = 2.0 * eta / sqrt(PI_D);
-  const double xi = pos[3 * i], yi = pos[3 * i + 1], zi_ = pos[3 * i + 2];
-  double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (long long w = tid; w < total; w += nthr) {
-    const int j = (int)(w % p.nion);
-    long long img = w / p.nion;
-    const int c = (int)(img % nc) - p.nimg[2];
-    img /= nc;
-    const int b = (int)(img % nb) - p.nimg[1];
-    const int a = (int)(img / nb) - p.nimg[0];
-    double d[3];
-    d[0] = pos[3 * j] + p.A[0][0] * a + p.A[0][1] * b + p.A[0][2] * c - xi;
-    d[1] = pos[3 * j + 1] + p.A[1][0] * a + p.A[1][1] * b + p.A[1][2] * c - yi;
-    d[2] = pos[3 * j + 2] + p.A[2][0] * a + p.A[2][1] * b + p.A[2][2] * c - zi_;
-    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    if (r2 < 1e-24 || r2 >= rc2) continue;
-    const double r = sqrt(r2);
-    const double ec = erfc(eta * r) / r;
-    const double fp = -ec / r - c2 * exp(-eta * eta * r2) / r;
-    sym_add(v + 1, d, 0.5 * z[i] * z[j] * fp / r);
-  }
-  block_sum<7>(red, v, tid, nthr, out7);
-}
-
-// out7 = (plane m's reciprocal energy, the six components of
-// sum (2 pi / vol) exp(-G^2/4eta^2)/G^2 |S(G)|^2 2 (1/4eta^2 + 1/G^2) G_a G_b).
-HD void ewald_plane_stress_block(const EwaldPar& p, const double* frac, const double* z, int m, int tid, int nthr,
-                                 double* red, double* out7) {
-  const int nm3 = 2 * p.ng[2] + 1, plane = ewald_plane_size(p);
-  const int m1 = m - p.ng[0];
-  const double gc2 = p.gcut * p.gcut, e4 = 4.0 * p.eta * p.eta;
-  double v[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int w = tid; w < plane; w += nthr) {
-    const int m2 = w / nm3 - p.ng[1], m3 = w % nm3 - p.ng[2];
-    double G[3];
-    const double g2 = ewald_g(p, m1, m2, m3, G);
-    if ((m1 == 0 && m2 == 0 && m3 == 0) || g2 > gc2) continue;
-    double sr = 0.0, si = 0.0;
-    for (int i = 0; i < p.nion; ++i) {
-      const double ph = 2.0 * PI_D * (m1 * frac[3 * i] + m2 * frac[3 * i + 1] + m3 * frac[3 * i + 2]);
-      sr += z[i] * cos(ph);
-      si += z[i] * sin(ph);
-    }
-    const double c = 2.0 * PI_D / p.vol * exp(-g2 / e4) / g2 * (sr * sr + si * si);
-    v[0] += c;
-    sym_add(v + 1, G, c * 2.0 * (1.0 / e4 + 1.0 / g2));
-  }
-  block_sum<7>(red, v, tid, nthr, out7);
-}
-
 #if !defined(OFDFT_EMU)
 __global__ void __launch_bounds__(128) k_stress_sf(const SlotDev* sd, const IonStencil* st, cx<double>* sf) {
   const SlotDev& s = *sd;
@@ -370,7 +330,9 @@ __global__ void __launch_bounds__(128) k_stress_sf(const SlotDev* sd, const IonS
 template <typename T>
 __global__ void __launch_bounds__(128) k_stress(const SlotDev* sd, StressArgs sa, double* out) {
   __shared__ double red[NSC * 128];
-  stress_block<T>(*sd, sa, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x, red, out + (size_t)NSC * blockIdx.x);
+  __shared__ cx<double> prod[STRESS_CHUNK];
+  stress_block<T>(*sd, sa, blockIdx.x, gridDim.x, threadIdx.x, blockDim.x, prod, red,
+                  out + (size_t)NSC * blockIdx.x);
 }
 template <typename T>
 __global__ void __launch_bounds__(256) k_rho_vxc(const T* rho, long long n, double* out) {
@@ -386,16 +348,6 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_scale(T* v, long long n, double f) {
   for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
     v[k] = (T)((double)v[k] * f);
-}
-__global__ void __launch_bounds__(128) k_ewald_real_stress(EwaldPar p, const double* pos, const double* z,
-                                                           double* out7) {
-  __shared__ double red[7 * 128];
-  ewald_real_stress_block(p, pos, z, blockIdx.x, threadIdx.x, blockDim.x, red, out7 + 7 * blockIdx.x);
-}
-__global__ void __launch_bounds__(128) k_ewald_plane_stress(EwaldPar p, const double* frac, const double* z,
-                                                            double* out7) {
-  __shared__ double red[7 * 128];
-  ewald_plane_stress_block(p, frac, z, blockIdx.x, threadIdx.x, blockDim.x, red, out7 + 7 * blockIdx.x);
 }
 #endif
 
