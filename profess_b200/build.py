@@ -10,9 +10,11 @@ Usage: python -m profess_b200.build [cuda|emu|all]
 """
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -23,15 +25,18 @@ EMU_DIR = os.path.join(ROOT, "tests", "_emu")
 LIB_PATH = os.path.join(LIB_DIR, "libprofess_b200.so")
 EMU_PATH = os.path.join(EMU_DIR, "libprofess_b200_emu.so")
 
-SOURCES = ["engine.cu"]
-HEADERS = ["cx.cuh", "fft.cuh", "dcsrch.cuh", "slot.cuh", "ntn_ctl.cuh", "passes.cuh", "setup.cuh", "ewald.cuh", "stress.cuh"]
+# engine.cu and, one unit per pass and precision, the pass kernels
+PASS_UNITS = ["pass_%s_%s.cu" % (p, t) for t in ("f64", "f32") for p in ("yzg", "yz", "split", "xfwd", "xinv")]
+SOURCES = ["engine.cu"] + PASS_UNITS
+HEADERS = ["kernels.cuh", "cx.cuh", "fft.cuh", "dcsrch.cuh", "slot.cuh", "ntn_ctl.cuh", "passes.cuh", "setup.cuh", "ewald.cuh", "stress.cuh"] + [
+    "f32/%s.cuh" % h for h in ("kernels", "cx", "fft", "dcsrch", "slot", "ntn_ctl", "passes")]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-Xcompiler", "-fPIC", "-shared",
-    "--expt-relaxed-constexpr", "-split-compile=0",
-    "-Xcompiler", "-fopenmp", "-lgomp",
+    "-Xcompiler", "-fPIC",
+    "--expt-relaxed-constexpr",
+    "-Xcompiler", "-fopenmp",
 ]
 
 
@@ -51,14 +56,31 @@ def _stale(target: str) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def build_cuda(force: bool = False, extra=None) -> str:
-    if not force and not _stale(LIB_PATH):
-        return LIB_PATH
-    os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [_nvcc()] + NVCC_FLAGS + (extra or []) + ["-I", INCLUDE, "-I", CSRC]
-    cmd += [os.path.join(CSRC, s) for s in SOURCES] + ["-o", LIB_PATH]
-    subprocess.run(cmd, check=True)
-    return LIB_PATH
+def build_cuda(force: bool = False, extra=None, lib: str = LIB_PATH, csrc: str = CSRC, log: str | None = None) -> str:
+    """Compile the units side by side and link them into ``lib`` (``extra``:
+    more nvcc flags; ``log``: a file for the compilers' output)."""
+    if not force and not _stale(lib):
+        return lib
+    os.makedirs(os.path.dirname(lib), exist_ok=True)
+    tmp = tempfile.TemporaryDirectory()
+    objs = [os.path.join(tmp.name, s[:-3] + ".o") for s in SOURCES]
+
+    def compile_unit(src, obj):
+        cmd = [_nvcc()] + NVCC_FLAGS + (extra or []) + ["-I", INCLUDE, "-I", csrc, "-c", os.path.join(csrc, src), "-o", obj]
+        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if r.returncode:
+            raise RuntimeError("%s\n%s" % (" ".join(cmd), r.stdout))
+        return r.stdout
+
+    with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        out = list(pool.map(compile_unit, SOURCES, objs))
+    if log:
+        with open(log, "w") as fh:
+            fh.write("".join(out))
+    subprocess.run([_nvcc(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fopenmp"] + objs +
+                   ["-lgomp", "-o", lib], check=True)
+    tmp.cleanup()
+    return lib
 
 
 def build_emu(force: bool = False) -> str:

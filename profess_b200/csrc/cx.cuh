@@ -48,6 +48,29 @@ template <typename T> HD cx<T> mul_i(cx<T> a, int dir) {
   return dir > 0 ? mk<T>(-a.y, a.x) : mk<T>(a.y, -a.x);
 }
 
+// Two adjacent complex values: one 16-byte access in FP32 (p must then be
+// 16-byte aligned), two in FP64.
+template <typename T> struct Cx2 { cx<T> a, b; };
+template <typename T> HD Cx2<T> ld_cx2(const cx<T>* p) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (sizeof(T) == 4) {
+    const float4 q = *(const float4*)p;
+    return Cx2<T>{mk<T>(q.x, q.y), mk<T>(q.z, q.w)};
+  }
+#endif
+  return Cx2<T>{p[0], p[1]};
+}
+template <typename T> HD void st_cx2(cx<T>* p, cx<T> a, cx<T> b) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (sizeof(T) == 4) {
+    *(float4*)p = make_float4(a.x, a.y, b.x, b.y);
+    return;
+  }
+#endif
+  p[0] = a;
+  p[1] = b;
+}
+
 // Precision-generic math wrappers (float versions map to the float library calls).
 HD double m_sqrt(double v) { return sqrt(v); }
 HD float m_sqrt(float v) { return sqrtf(v); }
@@ -61,69 +84,43 @@ HD float m_log(float v) { return logf(v); }
 HD double m_rcbrt(double v) { return rcbrt(v); }
 HD float m_rcbrt(float v) { return rcbrtf(v); }
 HD double m_rsqrt(double v) { return rsqrt(v); }
-HD float m_rsqrt(float v) { return rsqrtf(v); }
 #else
 HD double m_rcbrt(double v) { return 1.0 / cbrt(v); }
 HD float m_rcbrt(float v) { return 1.0f / cbrtf(v); }
 HD double m_rsqrt(double v) { return 1.0 / sqrt(v); }
-HD float m_rsqrt(float v) { return 1.0f / sqrtf(v); }
 #endif
 
-// ------------------------------------------------------------ async staging
-// Asynchronous global -> shared copies (cp.async) of n bytes by the threads of
-// a block: 16-byte copies when both addresses are 16-byte aligned and n is a
-// multiple of 16, else copies of the element size (4 or 8 bytes, which must
-// divide both addresses and n).  They put a block's input rows in flight at
-// once instead of one dependent load per work item.  cp_async_wait() waits
-// for the calling thread's copies; a block barrier after it makes every
-// thread's copies visible.  The host emulation copies at once.
-HD void cp_async_block(void* dst, const void* src, size_t n, int elem, int tid, int nthr) {
+// a^(-1/3) of a in [1e-30, 1e30] (icbrt_out says when it is not: the caller
+// then takes m_icbrt_any, once for a whole group of values, so that the fast
+// path is free of branches).  A single-precision seed y (exp2 of -log2(a)/3 of
+// the float with a's leading bits; relative error about 1e-6) and one step of
+// the series of (1 - e)^(-1/3), e = 1 - a y^3: y (1 + e/3 + 2 e^2/9) (the next
+// term is below 1e-17).  Largest relative error over [1e-5, 10] 1.5e-16
+// (rcbrt: 1.1e-16); with the seed by conversions 47 cycles a warp against 71,
+// by bits fewer.
+HD bool icbrt_out(double a) { return !(a >= 1e-30 && a <= 1e30); }
 #if defined(__CUDA_ARCH__)
-  const unsigned sdst = (unsigned)__cvta_generic_to_shared(dst);
-  const char* g = (const char*)src;
-  if (((((size_t)g) | sdst | n) & 15) == 0) {
-    for (size_t o = (size_t)tid * 16; o < n; o += (size_t)nthr * 16)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst + (unsigned)o), "l"(g + o) : "memory");
-  } else if (elem == 8) {
-    for (size_t o = (size_t)tid * 8; o < n; o += (size_t)nthr * 8)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sdst + (unsigned)o), "l"(g + o) : "memory");
-  } else {
-    for (size_t o = (size_t)tid * 4; o < n; o += (size_t)nthr * 4)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sdst + (unsigned)o), "l"(g + o) : "memory");
-  }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
+__device__ __forceinline__ float icbrt_seed(float a) {
+  float s = -0.333333343f * __log2f(a);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(s));
+  return s;
+}
+#endif
+HD double m_icbrt(double a) {
+#if defined(__CUDA_ARCH__)
+  const int h = ((__double2hiint(a) - 0x38000000) << 3) | (int)((unsigned)__double2loint(a) >> 29);
+  const int b = __float_as_int(icbrt_seed(__int_as_float(h)));
+  const double y = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+  const double e = fma(-(a * y), y * y, 1.0);
+  return fma(y * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y);
 #else
-  (void)elem;
-  (void)nthr;
-  if (tid == 0) memcpy(dst, src, n);
+  return 1.0 / cbrt(a);
 #endif
 }
-
-// One asynchronous copy of U = 4, 8 or 16 bytes (both addresses U-aligned);
-// cp_async_commit() closes the calling thread's group of copies.
-template <int U>
-HD void cp_async_unit(void* dst, const void* src) {
 #if defined(__CUDA_ARCH__)
-  const unsigned sdst = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (U == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sdst), "l"(src), "n"(U) : "memory");
+__device__ __noinline__ inline double m_icbrt_any(double a) { return rcbrt(a); }
 #else
-  memcpy(dst, src, U);
+HD double m_icbrt_any(double a) { return 1.0 / cbrt(a); }
 #endif
-}
-
-HD void cp_async_commit() {
-#if defined(__CUDA_ARCH__)
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-#endif
-}
-
-HD void cp_async_wait() {
-#if defined(__CUDA_ARCH__)
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-#endif
-}
 
 }  // namespace ofdft

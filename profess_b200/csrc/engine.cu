@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "kernels.cuh"
 #include "setup.cuh"
 #include "ewald.cuh"
 #include "stress.cuh"
@@ -69,53 +70,69 @@ static int d2h(void* h, const void* d, size_t n) { return cuda_check(cudaMemcpy(
 static int dsync() { return cuda_check(cudaDeviceSynchronize(), "synchronize"); }
 #endif
 
-// Row pairs per x-pass block.  The x passes keep their nf*rp complex columns
-// interleaved in shared memory ([x][column]), and their prologue and epilogue
-// walk x across the threads of a warp, so consecutive threads are nf*rp
-// complex values apart.  In FP64 an even count puts 2, 4 or 8 threads of a
-// quarter-warp on the same banks (8-way at nf*rp = 24); an odd count spreads
-// them over all 32 banks.  With an odd field count, one row pair fewer makes
-// the count odd: -2 % FP64 evaluation time at 96^3.  (In FP32 the same
-// change costs 2 %: the x passes there are bound by issue, not by banks.)
-static int odd_columns(int nf, int rp, size_t csz) {
-  return (csz == 16 && (nf & 1) && !(rp & 1) && rp > 1) ? rp - 1 : rp;
-}
-
 // Launch shape of a slot's passes: row pairs per x-forward task (*rp1) and
-// per x-inverse task (s.rp), up to OFDFT_XPASS_POINTS / n1 of them, whose
-// transform buffers (every field or ion species; the x-forward pass adds its
-// staged input rows) fit OFDFT_XFWD_KB32 / OFDFT_XINV_KB32 (FP32) or
-// OFDFT_XPASS_KB64 (FP64) KB of shared memory; and the tiles of the split y/z
-// path: z columns per y-pass task (*ty: columns of n2 values at an odd row
-// pitch) and y columns per z-pass task (*tz: a group of gmax fields of n3
-// values each), each in about 48 KB, at least 32 columns when n allows.
-// s needs n1..n3, k1, nf and kinetic; csz is the size of one complex value.
-#ifndef OFDFT_XFWD_KB32
-#define OFDFT_XFWD_KB32 48
+// per x-inverse task (s.rp), 32 at most, whose transform buffers (every field
+// or ion species) fit the KB of shared memory below, and the tiles of the
+// split y/z path: z columns per y-pass task (*ty: columns of n2 values at an
+// odd row pitch) and y columns per z-pass task (*tz: a group of gmax fields of
+// zh values each), each in about 48 KB, at least 32 and 16 columns when n
+// allows (160 x 160 x 256 WGC FP64: 16 columns of a z task 340 us, 32 570).
+// Cells too small for 148 tasks of that size still take 24 row pairs (16 x
+// 32^3 FP64: 12 + 18 us; every task is a fixed chain of latencies, so more and
+// smaller ones cost more than they spread).  s needs n1..n3, k1, nf, kinetic
+// and the plans; csz is the size of one complex value.
+//
+// The FP64 x passes live off resident warps: three 256-thread blocks (16 x
+// 96^3: forward 248 us with 74-78 KB and radices up to 8, 276 with radices up
+// to 12; inverse 368-370 with 56-74 KB; with two blocks of 110 KB at 128
+// registers 303 and 457).
+#ifndef OFDFT_XF_KB64
+#define OFDFT_XF_KB64 78
 #endif
-#ifndef OFDFT_XINV_KB32
-#define OFDFT_XINV_KB32 48
+#ifndef OFDFT_XI_KB64
+#define OFDFT_XI_KB64 56
 #endif
-#ifndef OFDFT_XPASS_KB64
-#define OFDFT_XPASS_KB64 72
+#ifndef OFDFT_X_THREADS
+#define OFDFT_X_THREADS 256
 #endif
-#ifndef OFDFT_XPASS_POINTS
-#define OFDFT_XPASS_POINTS 2048
+constexpr int X_THREADS = OFDFT_X_THREADS;  // threads of an x-pass block
+// Units of an x task of rp row pairs (at least one).
+static int x_units(const SlotDev& s, int rp) { return std::max(1, rp / s.zs); }
+// The FP32 passes (f32/) have a shape rule of their own: 256-thread blocks, row
+// pairs whose buffers (forward: and the staged rows of the two inputs) fit 48
+// KB, up to 2048 points.  The host emulation runs the FP64 passes' code.
+static size_t f32_xfwd_smem(int n1, int nfb, int nb, size_t esz) {
+  return align16((size_t)nfb * nb * n1 * 2 * esz) + 2 * align16((size_t)2 * nb * n1 * esz);
+}
+static size_t f32_xinv_smem(int n1, int nfb, int nb, size_t esz) {
+  return align16((size_t)nfb * nb * n1 * 2 * esz) + NCH * 33 * sizeof(double);
+}
+static size_t xf_smem(const SlotDev& s, int nfb, int rp, size_t esz) {
+#if !defined(OFDFT_EMU)
+  if (esz == 4) return f32_xfwd_smem(s.n1, nfb, rp, esz);
 #endif
+  return xfwd_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
+}
+static size_t xi_smem(const SlotDev& s, int nfb, int rp, size_t esz) {
+#if !defined(OFDFT_EMU)
+  if (esz == 4) return f32_xinv_smem(s.n1, nfb, rp, esz);
+#endif
+  return xinv_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
+}
 static void launch_shape(SlotDev& s, size_t csz, int nfx, int* rp1, int* ty, int* tz) {
   const size_t esz = csz / 2;
-  const size_t fkb = (size_t)(csz == 8 ? OFDFT_XFWD_KB32 : OFDFT_XPASS_KB64) * 1024;
-  const size_t ikb = (size_t)(csz == 8 ? OFDFT_XINV_KB32 : OFDFT_XPASS_KB64) * 1024;
-  *rp1 = std::max(1, std::min(32, OFDFT_XPASS_POINTS / s.n1));
-  while (*rp1 > 1 && xfwd_smem(s.n1, nfx, *rp1, esz) > fkb) (*rp1)--;
-  s.rp = std::max(1, std::min(32, OFDFT_XPASS_POINTS / s.n1));
-  while (s.rp > 1 && xinv_smem(s.n1, s.nf, s.rp, esz) > ikb) s.rp--;
-  *rp1 = odd_columns(s.nf, *rp1, csz);
-  s.rp = odd_columns(s.nf, s.rp, csz);
+  const bool f32 = csz == 8;
+  const int nrp = (s.n2 * s.n3 + 1) / 2;
+  const int most = f32 ? std::max(1, std::min(32, 2048 / s.n1)) : std::max(24, std::min(32, (nrp + 147) / 148));
+  const size_t fkb = (f32 ? 48 : OFDFT_XF_KB64) * 1024, ikb = (f32 ? 48 : OFDFT_XI_KB64) * 1024;
+  *rp1 = most;
+  while (*rp1 > s.zs && xf_smem(s, nfx, *rp1, esz) > fkb) (*rp1)--;
+  s.rp = most;
+  while (s.rp > s.zs && xi_smem(s, s.nf, s.rp, esz) > ikb) s.rp--;
   const int gmax = s.kinetic == KIN_WGC ? 3 : 1;
-  const size_t ycol = (size_t)(s.n2 | 1) * csz, zcol = (size_t)gmax * s.n3 * csz;
+  const size_t ycol = (size_t)(s.n2 | 1) * csz, zcol = (size_t)gmax * s.zh * csz;
   *ty = (int)std::max<size_t>(1, std::min<size_t>(s.n3, std::max<size_t>(48 * 1024 / ycol, 32)));
-  *tz = (int)std::max<size_t>(1, std::min<size_t>(s.n2, std::max<size_t>(48 * 1024 / zcol, 32)));
+  *tz = (int)std::max<size_t>(1, std::min<size_t>(s.n2, std::max<size_t>(48 * 1024 / zcol, f32 ? 32 : 16)));
   while (*ty > 1 && *ty * ycol > 160 * 1024) (*ty)--;
   while (*tz > 1 && *tz * zcol > 160 * 1024) (*tz)--;
 }
@@ -124,11 +141,11 @@ static void launch_shape(SlotDev& s, size_t csz, int nfx, int* rp1, int* ty, int
 // the largest plane it takes (one block of up to 226 KB per SM: fused at
 // 222 KB, a WGC 96^3 FP32 group ran 8 % faster than on the split path);
 // bigger planes run the split y/z path.
-static size_t yz_smem(const SlotDev& s, size_t csz) { return (size_t)s.n3 * (s.n2 | 1) * csz; }
+static size_t yz_smem(const SlotDev& s, size_t csz) { return (size_t)s.zh * (s.n2 | 1) * csz; }
 // A WGC slot's fused pass holds the three planes of a WGC group at once
 // (interleaved along y, odd pitch of 3*n2).
 static size_t yz_smem_slot(const SlotDev& s, size_t csz) {
-  return s.kinetic == KIN_WGC ? (size_t)s.n3 * ((3 * s.n2) | 1) * csz : yz_smem(s, csz);
+  return s.kinetic == KIN_WGC ? (size_t)s.zh * ((3 * s.n2) | 1) * csz : yz_smem(s, csz);
 }
 constexpr size_t YZ_SMEM_MAX = 226 * 1024;
 // Planes up to this size run 256-thread blocks (three per SM up to 75 KB, two
@@ -136,6 +153,12 @@ constexpr size_t YZ_SMEM_MAX = 226 * 1024;
 // blocks beat one 512-thread block on 84-99 KB plane sets (WT 72^3 FP64,
 // 108^3 FP32, WGC 64^3 FP32: 9-11 % faster evaluations).
 constexpr size_t YZ_SMEM_SMALL = 112 * 1024;
+// Threads of a block of the small class: about one per butterfly of radix 8
+// (a stage's work items), 64 to 192.  16 x 32^3 FP64: 30 us with 256 threads,
+// 19 with 128; 16 x 96^3 FP64: 345 with 256, 333 with 192, 370 with 128.
+static int yz_threads(const SlotDev& s) {
+  return std::max(64, std::min(192, (s.n2 * s.zh / 8 + 31) / 32 * 32));
+}
 
 // ------------------------------------------------------------ FFT plans
 static bool seven_smooth(int n) {
@@ -147,48 +170,85 @@ static bool seven_smooth(int n) {
 
 constexpr int MAX_N = 512;
 
+// Radix of the row split of a z axis of n points (passes.cuh), and the radix
+// sequence of the whole axis: the split's, then the default plan of the rest.
+// FP32 slots don't split: their solves end at the precision floor of the line
+// search, where another order of rounding moves one converged density in ten
+// by more than the FP32 resolution, so they keep the passes of f32/.
+static int z_split(int n, int prec) { return prec == OFDFT_FP64 && n % 2 == 0 && n >= 4 ? 2 : 1; }
+static int z_radices(int n, int prec, int rmax, int* rad) {
+  const int zs = z_split(n, prec);
+  if (zs == 1) return fft_radices(n, rmax, rad);
+  rad[0] = zs;
+  return 1 + fft_radices(n / zs, rmax, rad + 1);
+}
+
 // Radix caps the tuner may give an x-axis plan (the first is the default).
 static const int kCaps[2][3] = {{12, 8, 0}, {16, 12, 8}};  // [0] FP64, [1] FP32
+// The x-forward pass's own default cap: its last stage keeps two blocks of a
+// column in registers (16 x 96^3 FP64: 248 us, 276 with 12).
+static const int kXfwdCap[2] = {8, 16};
 
 struct PlanTable {
-  std::map<int, FftPlan> plans[2];  // [0] FP64 (OFDFT_FP64), [1] FP32: default radix cap
-  std::map<int, FftPlan> capped[2];  // key cap * 1024 + n: the plans of the other caps
-  void* d_tw64 = nullptr;           // exp(-2 pi i e / n), e < n, for every 7-smooth n <= MAX_N
+  std::map<int, StagePlan> plans[2];  // [0] FP64 (OFDFT_FP64), [1] FP32: default radix cap
+  std::map<int, StagePlan> zplan[2];   // whole z axis: the row split's radix, then the default plan of the rest
+  std::map<int, StagePlan> capped[2];  // key cap * 1024 + n: the plans of the other caps
+  void* d_tw64 = nullptr;           // stage twiddles of every plan (FftPlan::stw)
   void* d_tw32 = nullptr;
   int* d_idx = nullptr;             // perm and iperm of every plan
 
   int build() {
-    std::vector<long double> re, im;
-    std::map<int, int> root_off;
+    std::vector<long double> re, im;  // the twiddle table: stage tables of every plan
+    std::vector<int> idx;
     for (int n = 1; n <= MAX_N; ++n) {
       if (!seven_smooth(n)) continue;
-      root_off[n] = (int)re.size();
+      std::vector<long double> rr(n), ri(n);  // exp(-2 pi i e / n)
       for (int e = 0; e < n; ++e) {
         const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)e / (long double)n;
-        re.push_back(cosl(ang));
-        im.push_back(sinl(ang));
+        rr[e] = cosl(ang);
+        ri[e] = sinl(ang);
       }
-    }
-    std::vector<int> idx;
-    for (int pi = 0; pi < 2; ++pi)
-      for (int n = 1; n <= MAX_N; ++n) {
-        if (!seven_smooth(n)) continue;
+      const int root = (int)re.size();  // the roots themselves, then the plans' stage tables
+      re.insert(re.end(), rr.begin(), rr.end());
+      im.insert(im.end(), ri.begin(), ri.end());
+      if (n & 1) {
+        re.push_back(0.0L);
+        im.push_back(0.0L);
+      }
+      auto add = [&](const int* rad, int nst) {
+        StagePlan p;
+        memset((void*)&p, 0, sizeof(p));
+        p.root = root;
+        std::vector<int> perm(n), iperm(n);
+        fft_plan_fill(p, n, rad, nst, perm.data(), iperm.data());
+        const int end = fft_stage_twiddles(p, (int)re.size(), [&](int off, int j) {
+          if (off >= (int)re.size()) {
+            re.resize(off + 1, 0.0L);
+            im.resize(off + 1, 0.0L);
+          }
+          re[off] = rr[j];
+          im[off] = ri[j];
+        });
+        re.resize(end, 0.0L);
+        im.resize(end, 0.0L);
+        p.perm = (int)idx.size();
+        idx.insert(idx.end(), perm.begin(), perm.end());
+        p.iperm = (int)idx.size();
+        idx.insert(idx.end(), iperm.begin(), iperm.end());
+        return p;
+      };
+      for (int pi = 0; pi < 2; ++pi) {
+        int rad[FFT_MAX_STAGES];
         for (int ci = 0; ci < 3 && kCaps[pi][ci]; ++ci) {
-          int rad[FFT_MAX_STAGES];
           const int nst = fft_radices(n, kCaps[pi][ci], rad);
-          FftPlan p;
-          memset(&p, 0, sizeof(p));
-          std::vector<int> perm(n), iperm(n);
-          fft_plan_fill(p, n, rad, nst, perm.data(), iperm.data());
-          p.root = root_off[n];
-          p.perm = (int)idx.size();
-          idx.insert(idx.end(), perm.begin(), perm.end());
-          p.iperm = (int)idx.size();
-          idx.insert(idx.end(), iperm.begin(), iperm.end());
+          const StagePlan p = add(rad, nst);
           if (ci == 0) plans[pi][n] = p;
           else capped[pi][kCaps[pi][ci] * 1024 + n] = p;
         }
+        const int nst = z_radices(n, pi, kCaps[pi][0], rad);
+        zplan[pi][n] = add(rad, nst);
       }
+    }
     const size_t nt = re.size();
     std::vector<cx<double>> t64(nt);
     std::vector<cx<float>> t32(nt);
@@ -205,7 +265,7 @@ struct PlanTable {
     return rc;
   }
   // The plan of length n with radix cap cap (0 or the default cap: the default plan).
-  const FftPlan& get(int pi, int n, int cap) const {
+  const StagePlan& get(int pi, int n, int cap) const {
     auto it = capped[pi].find(cap * 1024 + n);
     return it == capped[pi].end() ? plans[pi].at(n) : it->second;
   }
@@ -231,54 +291,10 @@ enum Pass : int { P_VEC = 0, P_X1 = 1, P_Y2 = 2, P_Z3 = 3, P_Y4 = 4, P_X5 = 5, P
 constexpr int VEC_PER_TICK = 2;
 constexpr int VCHUNK = 4096;
 
-// Minimum resident 256-thread blocks per SM of the x and split y/z pass
-// kernels per precision (it caps their registers at 65536 / (256 * minb)).
-#ifndef OFDFT_MINB_FP32
-#define OFDFT_MINB_FP32 4
-#endif
-#ifndef OFDFT_MINB_FP64
-#define OFDFT_MINB_FP64 3
-#endif
-template <typename T> struct PassMinBlocks { static constexpr int value = OFDFT_MINB_FP32; };
-template <> struct PassMinBlocks<double> { static constexpr int value = OFDFT_MINB_FP64; };
-// The x-inverse pass (transform, then the real-space epilogue of two points
-// per work item) separately: its FP64 epilogue needs more registers.
-#ifndef OFDFT_XINV_MINB_FP64
-#define OFDFT_XINV_MINB_FP64 3
-#endif
-#ifndef OFDFT_XINV_MINB_FP32
-#define OFDFT_XINV_MINB_FP32 OFDFT_MINB_FP32
-#endif
-template <typename T> struct XinvMinBlocks { static constexpr int value = OFDFT_XINV_MINB_FP32; };
-template <> struct XinvMinBlocks<double> { static constexpr int value = OFDFT_XINV_MINB_FP64; };
-
 #if !defined(OFDFT_EMU)
 template <typename T> __global__ void __launch_bounds__(256) k_vec(Args<T> a) {
   extern __shared__ __align__(16) char sm[];
   vec_block<T>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-template <typename T, int KS> __global__ void __launch_bounds__(256, PassMinBlocks<T>::value) k_xfwd(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  xfwd_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-template <typename T> __global__ void __launch_bounds__(256, PassMinBlocks<T>::value) k_ypass(Args<T> a, int dir) {
-  extern __shared__ __align__(16) char sm[];
-  ypass_block<T>(a, blockIdx.x, threadIdx.x, blockDim.x, sm, dir);
-}
-template <typename T, int KS> __global__ void __launch_bounds__(256, PassMinBlocks<T>::value) k_zpass(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  zpass_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-// Fused y-z pass: 256-thread blocks, up to three per SM, for planes up to
-// YZ_SMEM_SMALL; 512-thread blocks, one per SM, for larger planes.
-template <typename T, int NT, int KS>
-__global__ void __launch_bounds__(NT, NT == 256 ? 3 : 1) k_yzpass(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  yzpass_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-template <typename T, int KS> __global__ void __launch_bounds__(256, XinvMinBlocks<T>::value) k_xinv(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  xinv_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
 }
 // keKernel planes from the reference layout (k1, n2, n3), x fastest, into
 // the engine's kx-major digit-reversed layout.
@@ -354,7 +370,8 @@ struct HostSlot {
   int prec = 0;
   SlotDev sd;
   std::vector<std::pair<void*, size_t>> allocs;  // device blocks and their sizes
-  int nrowpairs = 0, rp1 = 1;
+  int nunits = 0;               // units of the x passes: pairs of rows, with the row split two pairs each
+  int rp1 = 1;                  // row pairs per x-forward task
   int ty = 1, tz = 1;           // z columns per y-pass task and y columns per z-pass task (split path)
   int xcap = 0;                 // radix cap of the x-axis plan (0: the default)
   int yzt = 0;                  // threads of the fused y-z pass (0: by plane size)
@@ -618,6 +635,13 @@ struct Engine {
     return upload_slot(i);
   }
 
+  // The x plans of a slot (cap 0: the defaults).
+  void set_x_plans(SlotDev& s, int pi, int xcap) {
+    s.px = plans.get(pi, s.n1, xcap);
+    s.qx = x_plan(plans.get(pi, s.n1, xcap));
+    s.qxf = x_plan(plans.get(pi, s.n1, xcap ? xcap : kXfwdCap[pi]));
+  }
+
   int create_slot(const ofdft_cell_desc* d, int* out) {
     if (!d) return fail(OFDFT_EINVAL, "null descriptor");
     const int ns[3] = {d->n1, d->n2, d->n3};
@@ -641,9 +665,13 @@ struct Engine {
     s.N = (long long)d->n1 * d->n2 * d->n3;
     s.Nc = (long long)s.k1 * d->n2 * d->n3;
     const int pi = d->precision == OFDFT_FP32 ? 1 : 0;
-    s.px = plans.plans[pi][d->n1];
-    s.py = plans.plans[pi][d->n2];
+    set_x_plans(s, pi, 0);
+    s.py = s.qy = plans.plans[pi][d->n2];
+    s.zs = z_split(s.n3, h.prec);
+    s.zh = s.n3 / s.zs;
     s.pz = plans.plans[pi][d->n3];
+    s.qz = plans.zplan[pi][d->n3];
+    s.qzh = plans.plans[pi][s.zh];
     if (int rc = set_geometry(h, d->lattice)) {
       h.used = false;
       return rc;
@@ -677,11 +705,11 @@ struct Engine {
     }
     // launch geometry
     const long long nrows = (long long)s.n2 * s.n3;
-    h.nrowpairs = (int)((nrows + 1) / 2);
+    h.nunits = (int)((nrows / s.zs + 1) / 2);
     const size_t csz = 2 * elem_size(h.prec);
     launch_shape(s, csz, std::max(s.nf, MAX_SPECIES), &h.rp1, &h.ty, &h.tz);
     s.ntask[K_VEC] = (int)((s.N + VCHUNK - 1) / VCHUNK);
-    s.ntask[K_X5] = (h.nrowpairs + s.rp - 1) / s.rp;
+    s.ntask[K_X5] = (h.nunits + x_units(s, s.rp) - 1) / x_units(s, s.rp);
     // buffers
     const size_t es = elem_size(h.prec);
     int rc;
@@ -690,7 +718,7 @@ struct Engine {
     if ((rc = alloc(h, &s.vion, es * s.N))) { free_slot(idx); return rc; }
     if ((rc = alloc(h, &s.kern, es * s.Nc * h.nplanes))) { free_slot(idx); return rc; }
     if ((rc = alloc(h, &s.spec, 2 * es * s.Nc * s.nf))) { free_slot(idx); return rc; }
-    const int ntmax = std::max(s.ntask[K_VEC], h.nrowpairs);  // any x-inverse task size the tuner picks
+    const int ntmax = std::max(s.ntask[K_VEC], h.nunits);  // any x-inverse task size the tuner picks
     if ((rc = alloc(h, (void**)&s.partials, sizeof(double) * NCH * ntmax))) { free_slot(idx); return rc; }
     if ((rc = alloc(h, (void**)&s.hist, sizeof(HistEntry) * HIST_MAX))) { free_slot(idx); return rc; }
     auto tuned = tune_cache.find(tune_key(h));
@@ -1046,8 +1074,8 @@ struct Engine {
     std::vector<cx<double>> sf((size_t)nion * L);
     for (int k = 0; k < nion; ++k)
       for (int w = 0; w < L; ++w) sf[(size_t)k * L + w] = stress_sf_entry(s, h.stencils[k], w);
-    sa.permy = plans.d_idx + s.py.perm;
-    sa.permz = plans.d_idx + s.pz.perm;
+    sa.permy = plans.d_idx + s.qy.perm;
+    sa.permz = plans.d_idx + s.qz.perm;
     sa.sf = sf.data();
     sa.species = species.data();
     double red[NSC];
@@ -1066,8 +1094,8 @@ struct Engine {
     int* dspec = (int*)(scratch + sf_bytes + part_bytes);
     rc = h2d(dspec, species.data(), sizeof(int) * (size_t)nion);
     if (!rc) {
-      sa.permy = plans.d_idx + s.py.perm;
-      sa.permz = plans.d_idx + s.pz.perm;
+      sa.permy = plans.d_idx + s.qy.perm;
+      sa.permz = plans.d_idx + s.qz.perm;
       sa.sf = dsf;
       sa.species = dspec;
       k_stress_sf<<<nion, 128, 0, stream>>>(d_slots + i, h.d_stencil, dsf);
@@ -1628,8 +1656,8 @@ struct Engine {
     const SlotDev& s = h.sd;
     const size_t esz = elem_size(h.prec);
     if (c.rp1 < 1 || c.rp1 > 32 || c.rp < 1 || c.rp > 32) return false;
-    if (xfwd_smem(s.n1, std::max(s.nf, MAX_SPECIES), c.rp1, esz) > 200 * 1024) return false;
-    if (xinv_smem(s.n1, std::max(s.nf, MAX_SPECIES), c.rp, esz) > 200 * 1024) return false;
+    if (xf_smem(s, std::max(s.nf, MAX_SPECIES), c.rp1, esz) > 200 * 1024) return false;
+    if (xi_smem(s, std::max(s.nf, MAX_SPECIES), c.rp, esz) > 200 * 1024) return false;
     if (c.yzt != 0 && c.yzt != 256 && c.yzt != 512) return false;
     return true;
   }
@@ -1637,10 +1665,10 @@ struct Engine {
     SlotDev& s = h.sd;
     const int pi = h.prec == OFDFT_FP32 ? 1 : 0;
     h.xcap = c.xcap;
-    s.px = plans.get(pi, s.n1, c.xcap);
+    set_x_plans(s, pi, c.xcap);
     h.rp1 = c.rp1;
     s.rp = c.rp;
-    s.ntask[K_X5] = (h.nrowpairs + s.rp - 1) / s.rp;
+    s.ntask[K_X5] = (h.nunits + x_units(s, s.rp) - 1) / x_units(s, s.rp);
     h.yzt = c.yzt;
     dirty = true;
   }
@@ -1742,8 +1770,6 @@ struct Engine {
       return apply(best);
     };
     const int pi = h.prec == OFDFT_FP32 ? 1 : 0;
-    const SlotDev& s = h.sd;
-    const size_t csz = 2 * elem_size(h.prec);
     for (int ci = 1; ci < 3 && kCaps[pi][ci]; ++ci) {
       Shape c = best;
       c.xcap = kCaps[pi][ci];
@@ -1752,12 +1778,12 @@ struct Engine {
     const int base1 = best.rp1, base5 = best.rp;
     for (int r : {base1 / 2, (3 * base1) / 4, (3 * base1) / 2, 2 * base1}) {
       Shape c = best;
-      c.rp1 = odd_columns(s.nf, std::max(1, r), csz);
+      c.rp1 = std::max(1, r);
       if (c.rp1 != best.rp1 && (rc = trial(c))) return rc;
     }
     for (int r : {base5 / 2, (3 * base5) / 4, (3 * base5) / 2, 2 * base5}) {
       Shape c = best;
-      c.rp = odd_columns(s.nf, std::max(1, r), csz);
+      c.rp = std::max(1, r);
       if (c.rp != best.rp && (rc = trial(c))) return rc;
     }
     if (uses_yz(h))
@@ -1864,6 +1890,7 @@ struct Engine {
       for (int k = 0; k < NPASS; ++k) {
         lists[p][k].h.clear();
         lists[p][k].smem = 0;
+        lists[p][k].nthr = 0;
       }
     for (int i = 0; i < cap; ++i) {
       HostSlot& h = slots[i];
@@ -1876,17 +1903,18 @@ struct Engine {
       L[P_VEC].smem = std::max(L[P_VEC].smem, (size_t)(NCH * 33 * sizeof(double) + 16));
       const bool wgc = s.kinetic == KIN_WGC;
       const int px1 = wgc ? P_X1G : P_X1, pz3 = wgc ? P_Z3G : P_Z3, px5 = wgc ? P_X5G : P_X5;
-      for (int r = 0; r < h.nrowpairs; r += h.rp1)
-        L[px1].h.push_back({i, 0, r, std::min(h.rp1, h.nrowpairs - r)});
-      L[px1].nthr = 256;
-      L[px1].smem = std::max(L[px1].smem, xfwd_smem(s.n1, std::max(s.nf, s.ion.nspec), h.rp1, cs / 2));
+      const int u1 = x_units(s, h.rp1), u5 = x_units(s, s.rp);
+      for (int r = 0; r < h.nunits; r += u1) L[px1].h.push_back({i, 0, r, std::min(u1, h.nunits - r)});
+      L[px1].nthr = X_THREADS;
+      L[px1].smem = std::max(L[px1].smem, xf_smem(s, std::max(s.nf, s.ion.nspec), h.rp1, cs / 2));
       if (uses_yz(h)) {  // fused y-z pass: one task per (field, kx)
         const size_t sm = yz_smem_slot(s, cs);
         const bool big = h.yzt == 256 ? false : h.yzt == 512 ? true : sm > YZ_SMEM_SMALL;
         const int pyz = wgc ? (big ? P_YZBG : P_YZG) : (big ? P_YZB : P_YZ);
         for (int g = 0; g < s.ngroups; ++g)
-          for (int kx = 0; kx < s.k1; ++kx) L[pyz].h.push_back({i, g, kx, 0});
-        L[pyz].nthr = big ? 512 : 256;
+          for (int kx = 0; kx < s.k1; ++kx)
+            for (int hf = 0; hf < s.zs; ++hf) L[pyz].h.push_back({i, g, kx, hf});
+        L[pyz].nthr = big ? 512 : std::max(h.yzt ? h.yzt : h.prec == OFDFT_FP32 ? 256 : yz_threads(s), L[pyz].nthr);
         L[pyz].smem = std::max(L[pyz].smem, sm);
       } else {  // split path: y forward, z with the operator, y inverse
         for (int pass : {P_Y2, P_Y4}) {
@@ -1899,19 +1927,19 @@ struct Engine {
         }
         const int gmax = s.kinetic == KIN_WGC ? 3 : 1;
         for (int g = 0; g < s.ngroups; ++g)
-          for (int kx = 0; kx < s.k1; ++kx)
+          for (int kh = 0; kh < s.k1 * s.zs; ++kh)
             for (int t = 0; t < tile_count(s.n2, h.tz); ++t)
-              L[pz3].h.push_back({i, g, kx, tile_code(s.n2, h.tz, t)});
+              L[pz3].h.push_back({i, g, kh, tile_code(s.n2, h.tz, t)});
         L[pz3].nthr = 256;
-        L[pz3].smem = std::max(L[pz3].smem, (size_t)std::max(gmax, s.ion.nspec) * h.tz * s.n3 * cs);
+        L[pz3].smem = std::max(L[pz3].smem, (size_t)std::max(gmax, s.ion.nspec) * h.tz * s.zh * cs);
       }
       int ord = 0;
-      for (int r = 0; r < h.nrowpairs; r += s.rp) L[px5].h.push_back({i, r, std::min(s.rp, h.nrowpairs - r), ord++});
+      for (int r = 0; r < h.nunits; r += u5) L[px5].h.push_back({i, r, std::min(u5, h.nunits - r), ord++});
       L[P_CTL].h.push_back({i, 0, 0, 0});
       L[P_CTL].nthr = 64;
       L[P_CTL].smem = 0;
-      L[px5].nthr = 256;
-      L[px5].smem = std::max(L[px5].smem, xinv_smem(s.n1, std::max(s.nf, s.ion.nspec), s.rp, cs / 2));
+      L[px5].nthr = X_THREADS;
+      L[px5].smem = std::max(L[px5].smem, xi_smem(s, std::max(s.nf, s.ion.nspec), s.rp, cs / 2));
     }
 #if defined(OFDFT_EMU)
     for (int p = 0; p < 2; ++p)
@@ -2660,22 +2688,21 @@ static int scratch_address(int dev, char** base) {
 
 static size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Plan of length n (the engine's FP64 radix rule) with its roots of unity
+// Plan of length n (the engine's FP64 radix rule) with its stage twiddles
 // appended to tw at *toff and its digit-reversal tables to idx at *ioff (no
-// heap use).
-static void make_plan(int n, FftPlan& p, cx<double>* tw, int* toff, int* idx, int* ioff) {
-  memset(&p, 0, sizeof(p));
+// heap use).  A plan of a length up to 128 has at most 2 * 128 twiddles.
+constexpr int MAX_TW = 2 * MAX_DIM;
+static void make_plan(int n, bool z_axis, StagePlan& p, cx<double>* tw, int* toff, int* idx, int* ioff) {
+  memset((void*)&p, 0, sizeof(p));
   int rad[FFT_MAX_STAGES];
-  const int nst = fft_radices(n, FftMaxRadix<double>::value, rad);
+  const int nst = z_axis ? z_radices(n, OFDFT_FP64, FftMaxRadix<double>::value, rad) : fft_radices(n, FftMaxRadix<double>::value, rad);
   fft_plan_fill(p, n, rad, nst, idx + *ioff, idx + *ioff + n);
-  p.root = *toff;
   p.perm = *ioff;
   p.iperm = *ioff + n;
-  for (int e = 0; e < n; ++e) {
+  *toff = fft_stage_twiddles(p, *toff, [&](int off, int e) {
     const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)e / (long double)n;
-    tw[*toff + e] = mk<double>((double)cosl(a), (double)sinl(a));
-  }
-  *toff += n;
+    tw[off] = mk<double>((double)cosl(a), (double)sinl(a));
+  });
   *ioff += 2 * n;
 }
 }  // namespace noalloc
@@ -2708,12 +2735,18 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   s.k1 = d->n1 / 2 + 1;
   s.N = N;
   s.Nc = (long long)s.k1 * d->n2 * d->n3;
-  cx<double> tw[3 * MAX_DIM];  // roots of unity of the three plans
-  int ptab[6 * MAX_DIM];        // their digit-reversal tables
+  cx<double> tw[4 * MAX_TW];   // stage twiddles of the x, y, z and split-z plans
+  memset(tw, 0, sizeof(tw));
+  int ptab[8 * MAX_DIM];        // their digit-reversal tables
   int twoff = 0, poff = 0;
-  make_plan(d->n1, s.px, tw, &twoff, ptab, &poff);
-  make_plan(d->n2, s.py, tw, &twoff, ptab, &poff);
-  make_plan(d->n3, s.pz, tw, &twoff, ptab, &poff);
+  make_plan(d->n1, false, s.qx, tw, &twoff, ptab, &poff);
+  s.qx = x_plan(s.qx);
+  s.qxf = s.qx;
+  make_plan(d->n2, false, s.qy, tw, &twoff, ptab, &poff);
+  s.zs = z_split(s.n3, OFDFT_FP64);
+  s.zh = s.n3 / s.zs;
+  make_plan(d->n3, true, s.qz, tw, &twoff, ptab, &poff);
+  make_plan(s.zh, false, s.qzh, tw, &twoff, ptab, &poff);
   const double* L = d->lattice;
   auto A = [&](int r, int c) { return L[3 * c + r]; };
   const double det = A(0, 0) * (A(1, 1) * A(2, 2) - A(1, 2) * A(2, 1)) - A(0, 1) * (A(1, 0) * A(2, 2) - A(1, 2) * A(2, 0)) +
@@ -2744,17 +2777,18 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   const int kinds[4] = {G_HARTREE, G_KMUL, G_VW, G_KMUL};
   for (int g = 0; g < s.ngroups; ++g) { s.group_kind[g] = kinds[g]; s.group_f0[g] = g; s.group_nf[g] = 1; }
   const size_t cs = sizeof(cx<double>);
-  const int nrows = s.n2 * s.n3, nrp = (nrows + 1) / 2;
+  const int nrows = s.n2 * s.n3, nrp = (nrows / s.zs + 1) / 2;  // units
   int rp1 = 1, ty = 1, tz = 1;
   launch_shape(s, cs, s.nf, &rp1, &ty, &tz);  // the engine's own launch shape
-  s.ntask[K_X5] = (nrp + s.rp - 1) / s.rp;
+  const int u1 = x_units(s, rp1), u5 = x_units(s, s.rp);
+  s.ntask[K_X5] = (nrp + u5 - 1) / u5;
   s.buf[B_PHI] = (void*)rho;         // the input density (read only in EV_RHO mode)
   s.buf[B_W0] = (void*)potential;    // the output potential
   s.vion = (void*)ion_pot;
   // the engine's passes: the fused y-z pass when the plane fits, else the split path
   const size_t yzsm = yz_smem(s, cs);
   const bool fused = yzsm <= YZ_SMEM_MAX;
-  const int yzthr = yzsm <= YZ_SMEM_SMALL ? 256 : 512;
+  const int yzthr = yzsm <= YZ_SMEM_SMALL ? yz_threads(s) : 512;
   // task lists, packed one pass after the other: x forward, y forward (or
   // y-z), z, y inverse, x inverse, controller
   int nt[6] = {0, 0, 0, 0, 0, 0}, ntot = 0;
@@ -2765,20 +2799,21 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
     return true;
   };
   bool ok = true;
-  for (int r = 0; r < nrp && ok; r += rp1) ok = push(0, {0, 0, r, std::min(rp1, nrp - r)});
+  for (int r = 0; r < nrp && ok; r += u1) ok = push(0, {0, 0, r, std::min(u1, nrp - r)});
   if (fused) {
     for (int g = 0; g < s.ngroups && ok; ++g)
-      for (int kx = 0; kx < s.k1 && ok; ++kx) ok = push(1, {0, g, kx, 0});
+      for (int kx = 0; kx < s.k1 && ok; ++kx)
+        for (int hf = 0; hf < s.zs && ok; ++hf) ok = push(1, {0, g, kx, hf});
   } else {
     for (int f = 0; f < s.nf && ok; ++f)
       for (int kx = 0; kx < s.k1 && ok; ++kx)
         for (int t = 0; t < tile_count(s.n3, ty) && ok; ++t) ok = push(1, {0, f, kx, tile_code(s.n3, ty, t)});
     for (int g = 0; g < s.ngroups && ok; ++g)
-      for (int kx = 0; kx < s.k1 && ok; ++kx)
-        for (int t = 0; t < tile_count(s.n2, tz) && ok; ++t) ok = push(2, {0, g, kx, tile_code(s.n2, tz, t)});
+      for (int kh = 0; kh < s.k1 * s.zs && ok; ++kh)
+        for (int t = 0; t < tile_count(s.n2, tz) && ok; ++t) ok = push(2, {0, g, kh, tile_code(s.n2, tz, t)});
   }
   int ord = 0;
-  for (int r = 0; r < nrp && ok; r += s.rp) ok = push(3, {0, r, std::min(s.rp, nrp - r), ord++});
+  for (int r = 0; r < nrp && ok; r += u5) ok = push(3, {0, r, std::min(u5, nrp - r), ord++});
   if (ok) ok = push(4, {0, 0, 0, 0});
   if (!ok) return fail(OFDFT_EINVAL, "grid needs more tasks than the allocation-free evaluation holds");
   // scratch layout
@@ -2832,10 +2867,10 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   a.tw = (const cx<double>*)(base + o_tw);
   a.idx = didx;
   a.vchunk = VCHUNK;
-  const size_t sm1 = xfwd_smem(s.n1, s.nf, rp1, cs / 2);
+  const size_t sm1 = xfwd_smem(s.n1, s.nf, u1 * s.zs, cs / 2);
   const size_t sm2 = (size_t)ty * (s.n2 | 1) * cs;
-  const size_t sm3 = (size_t)tz * s.n3 * cs;
-  const size_t sm5 = xinv_smem(s.n1, s.nf, s.rp, cs / 2);
+  const size_t sm3 = (size_t)tz * s.zh * cs;
+  const size_t sm5 = xinv_smem(s.n1, s.nf, u5 * s.zs, cs / 2);
   auto attr = [&](auto kern, size_t sm) -> int {
     if (sm <= 48 * 1024) return OFDFT_OK;
     return cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
@@ -2843,16 +2878,16 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   };
   if ((rc = attr(k_xfwd<double, KS_WT>, sm1)) || (rc = attr(k_xinv<double, KS_WT>, sm5)))
     return rc;
-  if (fused && (rc = yzthr == 256 ? attr(k_yzpass<double, 256, KS_WT>, yzsm) : attr(k_yzpass<double, 512, KS_WT>, yzsm)))
+  if (fused && (rc = yzthr < 512 ? attr(k_yzpass<double, 256, KS_WT>, yzsm) : attr(k_yzpass<double, 512, KS_WT>, yzsm)))
     return rc;
   if (!fused && ((rc = attr(k_ypass<double>, sm2)) || (rc = attr(k_zpass<double, KS_WT>, sm3))))
     return rc;
   const Task* tb = (const Task*)(base + o_task);
   a.tasks = tb;
-  k_xfwd<double, KS_WT><<<nt[0], 256, sm1, st>>>(a);
+  k_xfwd<double, KS_WT><<<nt[0], X_THREADS, sm1, st>>>(a);
   a.tasks = tb + nt[0];
   if (fused) {
-    if (yzthr == 256) k_yzpass<double, 256, KS_WT><<<nt[1], 256, yzsm, st>>>(a);
+    if (yzthr < 512) k_yzpass<double, 256, KS_WT><<<nt[1], yzthr, yzsm, st>>>(a);
     else k_yzpass<double, 512, KS_WT><<<nt[1], 512, yzsm, st>>>(a);
   } else {
     k_ypass<double><<<nt[1], 256, sm2, st>>>(a, -1);
@@ -2862,7 +2897,7 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
     k_ypass<double><<<nt[1], 256, sm2, st>>>(a, 1);
   }
   a.tasks = tb + nt[0] + nt[1] + nt[2];
-  k_xinv<double, KS_WT><<<nt[3], 256, sm5, st>>>(a);
+  k_xinv<double, KS_WT><<<nt[3], X_THREADS, sm5, st>>>(a);
   a.tasks = tb + nt[0] + nt[1] + nt[2] + nt[3];
   k_ctl<double><<<1, 64, 0, st>>>(a, (int)K_X5);
   if ((rc = cuda_check(cudaGetLastError(), "kernel launch"))) return rc;

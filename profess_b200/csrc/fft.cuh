@@ -22,9 +22,11 @@
 // together: element i of column c lives at buf[c*cs + i*es]; work items
 // (column, butterfly) are spread over the block's threads with the column
 // fastest, so consecutive threads touch consecutive columns (conflict-free
-// shared-memory access when cs = 1, or when cs is odd).  The twiddles are
-// the n-th roots of unity exp(-2 pi i e / n), e < n, computed on the host in
-// long double; W_{L_s}^{e} is root[e n / L_s].  No scaling is applied.
+// shared-memory access when cs = 1, or when cs is odd).  The twiddles of
+// stage s are a table W_{L_s}^{j0 r} in the order the butterflies read them
+// (entry j0 R_s + r), computed on the host in long double: a butterfly's
+// R_s - 1 factors sit at fixed offsets from one address, two FP32 factors to
+// a 16-byte load.  No scaling is applied.
 #pragma once
 #include "cx.cuh"
 
@@ -45,9 +47,13 @@ struct FftPlan {
   int R[FFT_MAX_STAGES];
   int L[FFT_MAX_STAGES];               // block length of stage s, n / (R_0 ... R_{s-1})
   unsigned m_magic[FFT_MAX_STAGES];    // magic32(L[s] / R[s])
-  int root;                            // offset of exp(-2 pi i e / n), e < n, in the twiddle table
+  int root;                            // offset of exp(-2 pi i e / n), e < n, in the twiddle table (FP32 passes)
   int perm;                            // offset of perm (position -> frequency) in the index table
   int iperm;                           // offset of iperm (frequency -> position)
+};
+// A plan with its stage twiddle tables.
+struct StagePlan : FftPlan {
+  int stw[FFT_MAX_STAGES];             // offset (even) of stage s's twiddles W_{L_s}^{j0 r}, entry j0 R_s + r
 };
 
 // Exact quotient w / d for 0 <= w < 2^24 and 1 <= d <= 4096 from m32 = ceil(2^32 / d)
@@ -236,6 +242,7 @@ HD cx<T> twiddle_const(cx<T> x) {
 template <typename T, int R, int DIR> struct Dft;
 template <typename T, int A, int B, int DIR> HD void dft_ab(cx<T>* v);
 
+template <typename T, int DIR> struct Dft<T, 1, DIR> { static HD void run(cx<T>*) {} };
 template <typename T, int DIR> struct Dft<T, 2, DIR> { static HD void run(cx<T>* v) { dft2(v); } };
 template <typename T, int DIR> struct Dft<T, 3, DIR> { static HD void run(cx<T>* v) { dft3(v, DIR); } };
 template <typename T, int DIR> struct Dft<T, 4, DIR> { static HD void run(cx<T>* v) { dft4(v, DIR); } };
@@ -294,15 +301,55 @@ HD void dft_ab(cx<T>* v) {
   }
 }
 
+// v[r] *= w[r] (DIR < 0) or conj(w[r]) (DIR > 0), r = 1 .. R-1: a butterfly's
+// stage twiddles (w 16-byte aligned when R is even).
+template <typename T, int R, int DIR>
+HD void twiddle_mul(cx<T>* v, const cx<T>* __restrict__ w) {
+  if constexpr (sizeof(T) == 4 && R % 2 == 0) {
+#pragma unroll
+    for (int r = 0; r < R; r += 2) {
+      const Cx2<T> q = ld_cx2(w + r);
+      if (r > 0) v[r] = cmul(v[r], DIR < 0 ? q.a : conj(q.a));
+      v[r + 1] = cmul(v[r + 1], DIR < 0 ? q.b : conj(q.b));
+    }
+  } else {
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = cmul(v[r], DIR < 0 ? w[r] : conj(w[r]));
+  }
+}
+
+// f<R>() for the radix R of a stage: a switch over the radices a precision's
+// plans use.
+#define OFDFT_RADIX_CASE(r)                          \
+  case r:                                            \
+    if constexpr (r <= FftMaxRadix<T>::value) OFDFT_RADIX_DO(r); \
+    break;
+#define OFDFT_RADIX_SWITCH(R)  \
+  switch (R) {                 \
+    OFDFT_RADIX_CASE(2)        \
+    OFDFT_RADIX_CASE(3)        \
+    OFDFT_RADIX_CASE(4)        \
+    OFDFT_RADIX_CASE(5)        \
+    OFDFT_RADIX_CASE(6)        \
+    OFDFT_RADIX_CASE(7)        \
+    OFDFT_RADIX_CASE(8)        \
+    OFDFT_RADIX_CASE(9)        \
+    OFDFT_RADIX_CASE(10)       \
+    OFDFT_RADIX_CASE(12)       \
+    OFDFT_RADIX_CASE(14)       \
+    OFDFT_RADIX_CASE(15)       \
+    OFDFT_RADIX_CASE(16)       \
+    default: break;            \
+  }
+
 // One in-place stage of radix R over ncols columns (mcols = magic32(ncols)):
 // DIR = -1 forward (DFT, then twiddles), +1 inverse (conjugate twiddles,
-// then inverse DFT).  tstep = n / L.
+// then inverse DFT).  w: the stage's twiddles.
 template <typename T, int R, int DIR>
 HD void ip_stage_r(cx<T>* __restrict__ buf, int ncols, unsigned mcols, int cs, int es, int n, int L, unsigned mm,
-                   const cx<T>* __restrict__ roots, int tid, int nthr) {
+                   const cx<T>* __restrict__ wtab, int tid, int nthr) {
   const int m = L / R;
   const int total = (n / R) * ncols;
-  const int tstep = n / L;
   const int ms = m * es;
   for (int w = tid; w < total; w += nthr) {
     const int bf = magic_div32(w, mcols), c = w - bf * ncols;
@@ -311,48 +358,23 @@ HD void ip_stage_r(cx<T>* __restrict__ buf, int ncols, unsigned mcols, int cs, i
     cx<T> v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = p[r * ms];
-    const int e = j0 * tstep;
-    if (DIR > 0 && m > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], conj(roots[r * e]));
-    }
+    if (DIR > 0 && m > 1) twiddle_mul<T, R, DIR>(v, wtab + j0 * R);
     Dft<T, R, DIR>::run(v);
-    if (DIR < 0 && m > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], roots[r * e]);
-    }
+    if (DIR < 0 && m > 1) twiddle_mul<T, R, DIR>(v, wtab + j0 * R);
 #pragma unroll
     for (int r = 0; r < R; ++r) p[r * ms] = v[r];
   }
 }
 
 template <typename T, int DIR>
-HD void ip_stage(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const FftPlan& p, int s, const cx<T>* roots,
+HD void ip_stage(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const StagePlan& p, int s, const cx<T>* tw,
                  int tid, int nthr) {
-  constexpr int RM = FftMaxRadix<T>::value;
   const int n = p.n, L = p.L[s];
   const unsigned mm = p.m_magic[s];
-#define OFDFT_IP_CASE(r)                                                                          \
-  case r:                                                                                         \
-    if constexpr (r <= RM) ip_stage_r<T, r, DIR>(buf, ncols, mcols, cs, es, n, L, mm, roots, tid, nthr); \
-    break;
-  switch (p.R[s]) {
-    OFDFT_IP_CASE(2)
-    OFDFT_IP_CASE(3)
-    OFDFT_IP_CASE(4)
-    OFDFT_IP_CASE(5)
-    OFDFT_IP_CASE(6)
-    OFDFT_IP_CASE(7)
-    OFDFT_IP_CASE(8)
-    OFDFT_IP_CASE(9)
-    OFDFT_IP_CASE(10)
-    OFDFT_IP_CASE(12)
-    OFDFT_IP_CASE(14)
-    OFDFT_IP_CASE(15)
-    OFDFT_IP_CASE(16)
-    default: break;
-  }
-#undef OFDFT_IP_CASE
+  const cx<T>* w = tw + p.stw[s];
+#define OFDFT_RADIX_DO(r) ip_stage_r<T, r, DIR>(buf, ncols, mcols, cs, es, n, L, mm, w, tid, nthr)
+  OFDFT_RADIX_SWITCH(p.R[s])
+#undef OFDFT_RADIX_DO
 }
 
 // One stage whose inputs come from src.ld(c, i) and whose outputs go to
@@ -361,10 +383,9 @@ HD void ip_stage(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const Ff
 // last inverse stage store straight to it.
 template <typename T, int R, int DIR, class Src, class Dst>
 HD void ip_stage_io(const Src& src, const Dst& dst, int ncols, unsigned mcols, int n, int L, unsigned mm,
-                    const cx<T>* __restrict__ roots, int tid, int nthr) {
+                    const cx<T>* __restrict__ wtab, int tid, int nthr) {
   const int m = L / R;
   const int total = (n / R) * ncols;
-  const int tstep = n / L;
   for (int w = tid; w < total; w += nthr) {
     const int bf = magic_div32(w, mcols), c = w - bf * ncols;
     const int blk = magic_div32(bf, mm), j0 = bf - blk * m;
@@ -372,16 +393,9 @@ HD void ip_stage_io(const Src& src, const Dst& dst, int ncols, unsigned mcols, i
     cx<T> v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = src.ld(c, base + r * m);
-    const int e = j0 * tstep;
-    if (DIR > 0 && m > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], conj(roots[r * e]));
-    }
+    if (DIR > 0 && m > 1) twiddle_mul<T, R, DIR>(v, wtab + j0 * R);
     Dft<T, R, DIR>::run(v);
-    if (DIR < 0 && m > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], roots[r * e]);
-    }
+    if (DIR < 0 && m > 1) twiddle_mul<T, R, DIR>(v, wtab + j0 * R);
 #pragma unroll
     for (int r = 0; r < R; ++r) dst.st(c, base + r * m, v[r]);
   }
@@ -389,32 +403,14 @@ HD void ip_stage_io(const Src& src, const Dst& dst, int ncols, unsigned mcols, i
 
 // Stage s of plan p through accessors (a switch over the radix).
 template <typename T, int DIR, class Src, class Dst>
-HD void ip_stage_acc(const Src& src, const Dst& dst, int ncols, unsigned mcols, const FftPlan& p, int s,
-                     const cx<T>* roots, int tid, int nthr) {
-  constexpr int RM = FftMaxRadix<T>::value;
+HD void ip_stage_acc(const Src& src, const Dst& dst, int ncols, unsigned mcols, const StagePlan& p, int s,
+                     const cx<T>* tw, int tid, int nthr) {
   const int n = p.n, L = p.L[s];
   const unsigned mm = p.m_magic[s];
-#define OFDFT_IO_CASE(r)                                                                              \
-  case r:                                                                                             \
-    if constexpr (r <= RM) ip_stage_io<T, r, DIR>(src, dst, ncols, mcols, n, L, mm, roots, tid, nthr); \
-    break;
-  switch (p.R[s]) {
-    OFDFT_IO_CASE(2)
-    OFDFT_IO_CASE(3)
-    OFDFT_IO_CASE(4)
-    OFDFT_IO_CASE(5)
-    OFDFT_IO_CASE(6)
-    OFDFT_IO_CASE(7)
-    OFDFT_IO_CASE(8)
-    OFDFT_IO_CASE(9)
-    OFDFT_IO_CASE(10)
-    OFDFT_IO_CASE(12)
-    OFDFT_IO_CASE(14)
-    OFDFT_IO_CASE(15)
-    OFDFT_IO_CASE(16)
-    default: break;
-  }
-#undef OFDFT_IO_CASE
+  const cx<T>* w = tw + p.stw[s];
+#define OFDFT_RADIX_DO(r) ip_stage_io<T, r, DIR>(src, dst, ncols, mcols, n, L, mm, w, tid, nthr)
+  OFDFT_RADIX_SWITCH(p.R[s])
+#undef OFDFT_RADIX_DO
 }
 
 // The last forward stage (block length R, stride 1: no twiddles), a real
@@ -442,31 +438,12 @@ HD void ip_stage_op_r(cx<T>* __restrict__ buf, int ncols, unsigned mcols, int cs
 }
 
 template <typename T, class Op>
-HD void ip_stage_op(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const FftPlan& p, const Op& op, int tid,
+HD void ip_stage_op(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const StagePlan& p, const Op& op, int tid,
                     int nthr) {
-  constexpr int RM = FftMaxRadix<T>::value;
   const int n = p.n;
-#define OFDFT_OP_CASE(r)                                                                  \
-  case r:                                                                                 \
-    if constexpr (r <= RM) ip_stage_op_r<T, r>(buf, ncols, mcols, cs, es, n, op, tid, nthr); \
-    break;
-  switch (p.R[p.nst - 1]) {
-    OFDFT_OP_CASE(2)
-    OFDFT_OP_CASE(3)
-    OFDFT_OP_CASE(4)
-    OFDFT_OP_CASE(5)
-    OFDFT_OP_CASE(6)
-    OFDFT_OP_CASE(7)
-    OFDFT_OP_CASE(8)
-    OFDFT_OP_CASE(9)
-    OFDFT_OP_CASE(10)
-    OFDFT_OP_CASE(12)
-    OFDFT_OP_CASE(14)
-    OFDFT_OP_CASE(15)
-    OFDFT_OP_CASE(16)
-    default: break;
-  }
-#undef OFDFT_OP_CASE
+#define OFDFT_RADIX_DO(r) ip_stage_op_r<T, r>(buf, ncols, mcols, cs, es, n, op, tid, nthr)
+  OFDFT_RADIX_SWITCH(p.R[p.nst - 1])
+#undef OFDFT_RADIX_DO
 }
 
 // Full in-place transform of ncols columns (element i of column c at
@@ -476,17 +453,16 @@ HD void ip_stage_op(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, const
 // barrier), and the block synchronises after every stage, so the result is
 // complete on return.
 template <typename T, int DIR>
-HD void fft_inplace(cx<T>* buf, int ncols, int cs, int es, const FftPlan& p, const cx<T>* twtab, int tid, int nthr) {
+HD void fft_inplace(cx<T>* buf, int ncols, int cs, int es, const StagePlan& p, const cx<T>* tw, int tid, int nthr) {
   const unsigned mcols = magic32(ncols);
-  const cx<T>* roots = twtab + p.root;
   if (DIR < 0) {
     for (int s = 0; s < p.nst; ++s) {
-      ip_stage<T, -1>(buf, ncols, mcols, cs, es, p, s, roots, tid, nthr);
+      ip_stage<T, -1>(buf, ncols, mcols, cs, es, p, s, tw, tid, nthr);
       BLOCK_SYNC();
     }
   } else {
     for (int s = p.nst - 1; s >= 0; --s) {
-      ip_stage<T, 1>(buf, ncols, mcols, cs, es, p, s, roots, tid, nthr);
+      ip_stage<T, 1>(buf, ncols, mcols, cs, es, p, s, tw, tid, nthr);
       BLOCK_SYNC();
     }
   }
@@ -518,6 +494,37 @@ inline int fft_radices(int n, int rmax, int* out) {
     for (int b = a + 1; b < k; ++b)
       if (out[b] > out[a]) { const int t = out[a]; out[a] = out[b]; out[b] = t; }
   return k;
+}
+
+// Entries of the stage twiddle tables of a plan, and the tables themselves:
+// put(off, j) is called for every entry, whose value is exp(-2 pi i j / n).
+// Fills p.stw from off0 on (even offsets); a stage of stride 1 has no table.
+// Returns the end offset.
+template <class Put>
+inline int fft_stage_twiddles(StagePlan& p, int off0, Put put) {
+  int off = off0;
+  for (int s = 0; s < p.nst; ++s) {
+    const int m = p.L[s] / p.R[s];
+    p.stw[s] = off;
+    if (m == 1) continue;
+    for (int j0 = 0; j0 < m; ++j0)
+      for (int r = 0; r < p.R[s]; ++r) put(off + j0 * p.R[s] + r, (int)((long long)j0 * r % p.L[s] * (p.n / p.L[s])));
+    off += p.L[s] + (p.L[s] & 1);
+  }
+  return off;
+}
+
+// The x-axis plan of a length: the x passes fuse the first and the last
+// stage with their inputs and outputs, so a one-stage plan gets a second
+// stage of radix 1.
+inline StagePlan x_plan(StagePlan p) {
+  if (p.nst != 1) return p;
+  p.nst = 2;
+  p.R[1] = 1;
+  p.L[1] = 1;
+  p.m_magic[1] = magic32(1);
+  p.stw[1] = p.stw[0];
+  return p;
 }
 
 // Fill plan p of length n from its radix sequence (stage block lengths and

@@ -1,0 +1,5 @@
+#include "f32/kernels.cuh"
+namespace ofdft {
+template __global__ void k_yzpass<float, 256, KS_WGC>(Args<float>);
+template __global__ void k_yzpass<float, 512, KS_WGC>(Args<float>);
+}

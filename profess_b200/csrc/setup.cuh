@@ -193,8 +193,8 @@ HD void kernel_freq(const SlotDev& s, const int* idx, long long i, int& kx, int&
   kx = (int)(i / nrows);
   const int rem = (int)(i - (long long)kx * nrows);
   const int qz = rem / s.n2, qy = rem - qz * s.n2;
-  ky = idx[s.py.perm + qy];
-  kz = idx[s.pz.perm + qz];
+  ky = idx[s.qy.perm + qy];
+  kz = idx[s.qz.perm + qz];
 }
 
 // Index in the reference layout keKernel(k1G, k2G, k3G, plane) of element i

@@ -305,7 +305,8 @@ HD void rho_vxc_block(const T* rho, long long n, int b, int nblk, int tid, int n
     const double r = (double)rho[k];
     const double r13 = cbrt(r);
     double vxc, exc;
-    lda_point<double>(r, r13, 0.62035049089940009 / r13, vxc, exc);
+    const double rs = 0.62035049089940009 / r13;
+    lda_point<double>(r, r13, rs, sqrt(rs), vxc, exc);
     acc += r * vxc;
   }
   block_sum<1>(red, &acc, tid, nthr, out);
