@@ -1911,7 +1911,9 @@ struct Engine {
         const size_t sm = yz_smem_slot(s, cs);
         const bool big = h.yzt == 256 ? false : h.yzt == 512 ? true : sm > YZ_SMEM_SMALL;
         const int pyz = wgc ? (big ? P_YZBG : P_YZG) : (big ? P_YZB : P_YZ);
-        for (int g = 0; g < s.ngroups; ++g)
+        // the WGC groups of three fields (the last ones) first: the long tasks
+        // must not start in the launch's last wave
+        for (int g = s.ngroups - 1; g >= 0; --g)
           for (int kx = 0; kx < s.k1; ++kx)
             for (int hf = 0; hf < s.zs; ++hf) L[pyz].h.push_back({i, g, kx, hf});
         L[pyz].nthr = big ? 512 : std::max(h.yzt ? h.yzt : h.prec == OFDFT_FP32 ? 256 : yz_threads(s), L[pyz].nthr);

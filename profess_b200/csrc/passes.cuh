@@ -772,6 +772,8 @@ HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Pu
   }
 }
 
+template <int N> struct Count { static constexpr int value = N; };
+
 // Every field of a range of units in one block: element i of column f*nc +
 // col*nb + b at buf[i*es + f*nc + col*nb + b].
 template <typename T, int KS>
@@ -793,28 +795,52 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   const FieldPar<T> fp = field_par<T>(s);
   const unsigned mn1 = magic32(n1);
   const bool two = !in.rho_mode && in.cb != T(0);
-  // an input value, or a second row that is missing (zero)
-  auto load = [&](const T* __restrict__ A, int i, bool have) {
-    if (!have) return T(0);
-    if (ev == EV_ION || in.rho_mode) return A[i];
-    const T x = two ? phi_in(in.ca, A[i], in.cb, in.B[i]) : in.ca * A[i];
-    return ev == EV_FORCE ? x * x : x;
+  // the inputs of NP points at once: every load of both arrays first
+  auto inputs = [&](auto np, const T* __restrict__ A, const int* idx, bool has1, T* x) {
+    constexpr int NP = decltype(np)::value;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) x[k] = A[idx[k]];
+    if (ev != EV_ION && !in.rho_mode) {
+      if (two) {
+        T y[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) y[k] = in.B[idx[k]];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) x[k] = phi_in(in.ca, x[k], in.cb, y[k]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) x[k] *= in.ca;
+      }
+      if (ev == EV_FORCE) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) x[k] *= x[k];
+      }
+    }
+    if (!has1) {  // a missing second row is zero
+#pragma unroll
+      for (int k = 1; k < NP; k += 2) x[k] = T(0);
+    }
   };
   for (int f0 = 0; f0 < (ev == EV_ION ? nf : 1); ++f0) {
     const T* __restrict__ A = ev == EV_ION ? (const T*)s.buf[B_PHI + f0] : in.A;
+#pragma unroll 2
     for (int w = tid; w < nb * n1; w += nthr) {
       const int b = magic_div32(w, mn1), i = w - b * n1;
       const bool has1 = rm.has1(u0 + b);
-      const int i0 = rm.row(u0 + b, 0) * n1 + i;
+      const int i0 = rm.row(u0 + b, 0) * n1 + i, i1 = has1 ? i0 + n1 : i0;
       cx<T>* d = buf + i * es + b;
       if (zs == 1) {
-        const T x[2] = {load(A, i0, true), load(A, i0 + n1, has1)};
+        const int idx[2] = {i0, i1};
+        T x[2];
+        inputs(Count<2>(), A, idx, has1, x);
         auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], v[1]); };
         if (setup) put(f0, x);
         else point_fields<T, KS, 2>(fp, in.rho_mode, nf, x, put);
       } else {
-        const int i2 = i0 + rm.half * n1;
-        const T x[4] = {load(A, i0, true), load(A, i0 + n1, has1), load(A, i2, true), load(A, i2 + n1, has1)};
+        const int hs = rm.half * n1;
+        const int idx[4] = {i0, i1, i0 + hs, i1 + hs};
+        T x[4];
+        inputs(Count<4>(), A, idx, has1, x);
         auto put = [&](int f, const T* v) {
           d[f * nc] = mk<T>(add_rn(v[0], v[2]), add_rn(v[1], v[3]));
           d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), add_rn(v[1], -v[3]));
