@@ -795,8 +795,10 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   const FieldPar<T> fp = field_par<T>(s);
   const unsigned mn1 = magic32(n1);
   const bool two = !in.rho_mode && in.cb != T(0);
-  // the inputs of NP points at once: every load of both arrays first
-  auto inputs = [&](auto np, const T* __restrict__ A, const int* idx, bool has1, T* x) {
+  // the inputs of NP points at once: every load of both arrays first.  A
+  // missing second row has the first one's inputs (valid ones: the functional's
+  // powers of a zero density may be infinite), and put stores zero fields for it.
+  auto inputs = [&](auto np, const T* __restrict__ A, const int* idx, T* x) {
     constexpr int NP = decltype(np)::value;
 #pragma unroll
     for (int k = 0; k < NP; ++k) x[k] = A[idx[k]];
@@ -816,10 +818,6 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
         for (int k = 0; k < NP; ++k) x[k] *= x[k];
       }
     }
-    if (!has1) {  // a missing second row is zero
-#pragma unroll
-      for (int k = 1; k < NP; k += 2) x[k] = T(0);
-    }
   };
   for (int f0 = 0; f0 < (ev == EV_ION ? nf : 1); ++f0) {
     const T* __restrict__ A = ev == EV_ION ? (const T*)s.buf[B_PHI + f0] : in.A;
@@ -832,18 +830,18 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
       if (zs == 1) {
         const int idx[2] = {i0, i1};
         T x[2];
-        inputs(Count<2>(), A, idx, has1, x);
-        auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], v[1]); };
+        inputs(Count<2>(), A, idx, x);
+        auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], has1 ? v[1] : T(0)); };
         if (setup) put(f0, x);
         else point_fields<T, KS, 2>(fp, in.rho_mode, nf, x, put);
       } else {
         const int hs = rm.half * n1;
         const int idx[4] = {i0, i1, i0 + hs, i1 + hs};
         T x[4];
-        inputs(Count<4>(), A, idx, has1, x);
+        inputs(Count<4>(), A, idx, x);
         auto put = [&](int f, const T* v) {
-          d[f * nc] = mk<T>(add_rn(v[0], v[2]), add_rn(v[1], v[3]));
-          d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), add_rn(v[1], -v[3]));
+          d[f * nc] = mk<T>(add_rn(v[0], v[2]), has1 ? add_rn(v[1], v[3]) : T(0));
+          d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), has1 ? add_rn(v[1], -v[3]) : T(0));
         };
         if (setup) put(f0, x);
         else point_fields<T, KS, 4>(fp, in.rho_mode, nf, x, put);
