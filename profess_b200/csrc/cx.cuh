@@ -78,6 +78,15 @@ HD double m_cbrt(double v) { return cbrt(v); }
 HD float m_cbrt(float v) { return cbrtf(v); }
 HD double m_pow(double a, double b) { return pow(a, b); }
 HD float m_pow(float a, float b) { return powf(a, b); }
+// The power as a call, for a rare case: its code does not take registers from
+// the common one.
+#if defined(__CUDA_ARCH__)
+__device__ __noinline__ inline double m_pow_call(double a, double b) { return pow(a, b); }
+__device__ __noinline__ inline float m_pow_call(float a, float b) { return powf(a, b); }
+#else
+HD double m_pow_call(double a, double b) { return pow(a, b); }
+HD float m_pow_call(float a, float b) { return powf(a, b); }
+#endif
 HD double m_log(double v) { return log(v); }
 HD float m_log(float v) { return logf(v); }
 #if defined(__CUDA_ARCH__)

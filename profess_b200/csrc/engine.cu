@@ -185,12 +185,9 @@ static int z_radices(int n, int prec, int rmax, int* rad) {
 
 // Radix caps the tuner may give an x-axis plan (the first is the default).
 static const int kCaps[2][3] = {{12, 8, 0}, {16, 12, 8}};  // [0] FP64, [1] FP32
-// The x-forward pass's own default cap: its last stage keeps two blocks of a
-// column in registers (16 x 96^3 FP64: 248 us, 276 with 12).
-static const int kXfwdCap[2] = {8, 16};
-
 struct PlanTable {
   std::map<int, StagePlan> plans[2];  // [0] FP64 (OFDFT_FP64), [1] FP32: default radix cap
+  std::map<int, StagePlan> xfwd[2];    // x-forward pass
   std::map<int, StagePlan> zplan[2];   // whole z axis: the row split's radix, then the default plan of the rest
   std::map<int, StagePlan> capped[2];  // key cap * 1024 + n: the plans of the other caps
   void* d_tw64 = nullptr;           // stage twiddles of every plan (FftPlan::stw)
@@ -245,8 +242,8 @@ struct PlanTable {
           if (ci == 0) plans[pi][n] = p;
           else capped[pi][kCaps[pi][ci] * 1024 + n] = p;
         }
-        const int nst = z_radices(n, pi, kCaps[pi][0], rad);
-        zplan[pi][n] = add(rad, nst);
+        xfwd[pi][n] = add(rad, xfwd_radices(n, kCaps[pi][0], rad));
+        zplan[pi][n] = add(rad, z_radices(n, pi, kCaps[pi][0], rad));
       }
     }
     const size_t nt = re.size();
@@ -639,7 +636,7 @@ struct Engine {
   void set_x_plans(SlotDev& s, int pi, int xcap) {
     s.px = plans.get(pi, s.n1, xcap);
     s.qx = x_plan(plans.get(pi, s.n1, xcap));
-    s.qxf = x_plan(plans.get(pi, s.n1, xcap ? xcap : kXfwdCap[pi]));
+    s.qxf = plans.xfwd[pi].at(s.n1);
   }
 
   int create_slot(const ofdft_cell_desc* d, int* out) {
@@ -2690,14 +2687,18 @@ static int scratch_address(int dev, char** base) {
 
 static size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Plan of length n (the engine's FP64 radix rule) with its stage twiddles
-// appended to tw at *toff and its digit-reversal tables to idx at *ioff (no
-// heap use).  A plan of a length up to 128 has at most 2 * 128 twiddles.
+// Plan of length n (the engine's FP64 radix rule for its use) with its stage
+// twiddles appended to tw at *toff and its digit-reversal tables to idx at
+// *ioff (no heap use).  A plan of a length up to 128 has at most 2 * 128
+// twiddles.
 constexpr int MAX_TW = 2 * MAX_DIM;
-static void make_plan(int n, bool z_axis, StagePlan& p, cx<double>* tw, int* toff, int* idx, int* ioff) {
+enum PlanUse { FOR_AXIS, FOR_XFWD, FOR_WHOLE_Z };
+static void make_plan(int n, PlanUse use, StagePlan& p, cx<double>* tw, int* toff, int* idx, int* ioff) {
   memset((void*)&p, 0, sizeof(p));
   int rad[FFT_MAX_STAGES];
-  const int nst = z_axis ? z_radices(n, OFDFT_FP64, FftMaxRadix<double>::value, rad) : fft_radices(n, FftMaxRadix<double>::value, rad);
+  constexpr int rmax = FftMaxRadix<double>::value;
+  const int nst = use == FOR_XFWD ? xfwd_radices(n, rmax, rad)
+                  : use == FOR_WHOLE_Z ? z_radices(n, OFDFT_FP64, rmax, rad) : fft_radices(n, rmax, rad);
   fft_plan_fill(p, n, rad, nst, idx + *ioff, idx + *ioff + n);
   p.perm = *ioff;
   p.iperm = *ioff + n;
@@ -2737,18 +2738,18 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   s.k1 = d->n1 / 2 + 1;
   s.N = N;
   s.Nc = (long long)s.k1 * d->n2 * d->n3;
-  cx<double> tw[4 * MAX_TW];   // stage twiddles of the x, y, z and split-z plans
+  cx<double> tw[5 * MAX_TW];   // stage twiddles of the x (inverse, forward), y, z and split-z plans
   memset(tw, 0, sizeof(tw));
-  int ptab[8 * MAX_DIM];        // their digit-reversal tables
+  int ptab[10 * MAX_DIM];       // their digit-reversal tables
   int twoff = 0, poff = 0;
-  make_plan(d->n1, false, s.qx, tw, &twoff, ptab, &poff);
+  make_plan(d->n1, FOR_AXIS, s.qx, tw, &twoff, ptab, &poff);
   s.qx = x_plan(s.qx);
-  s.qxf = s.qx;
-  make_plan(d->n2, false, s.qy, tw, &twoff, ptab, &poff);
+  make_plan(d->n1, FOR_XFWD, s.qxf, tw, &twoff, ptab, &poff);
+  make_plan(d->n2, FOR_AXIS, s.qy, tw, &twoff, ptab, &poff);
   s.zs = z_split(s.n3, OFDFT_FP64);
   s.zh = s.n3 / s.zs;
-  make_plan(d->n3, true, s.qz, tw, &twoff, ptab, &poff);
-  make_plan(s.zh, false, s.qzh, tw, &twoff, ptab, &poff);
+  make_plan(d->n3, FOR_WHOLE_Z, s.qz, tw, &twoff, ptab, &poff);
+  make_plan(s.zh, FOR_AXIS, s.qzh, tw, &twoff, ptab, &poff);
   const double* L = d->lattice;
   auto A = [&](int r, int c) { return L[3 * c + r]; };
   const double det = A(0, 0) * (A(1, 1) * A(2, 2) - A(1, 2) * A(2, 1)) - A(0, 1) * (A(1, 0) * A(2, 2) - A(1, 2) * A(2, 0)) +

@@ -514,9 +514,8 @@ inline int fft_stage_twiddles(StagePlan& p, int off0, Put put) {
   return off;
 }
 
-// The x-axis plan of a length: the x passes fuse the first and the last
-// stage with their inputs and outputs, so a one-stage plan gets a second
-// stage of radix 1.
+// The x-inverse plan of a length: the pass runs at least two stages, so a
+// one-stage plan gets a second stage of radix 1.
 inline StagePlan x_plan(StagePlan p) {
   if (p.nst != 1) return p;
   p.nst = 2;
@@ -525,6 +524,30 @@ inline StagePlan x_plan(StagePlan p) {
   p.m_magic[1] = magic32(1);
   p.stw[1] = p.stw[0];
   return p;
+}
+
+// Radix sequence of the x-forward pass: the pass keeps two blocks of its last
+// stage in registers (x_last_split), so that stage's radix is 4 at most - or 1,
+// a stage that only splits the rows - whatever the others are.  At 80
+// registers a thread a radix of 5 or 6 spills 0.1 KB, 8 0.3 KB, 12 1.2 KB (16 x
+// 96^3 FP64: 258 us with 6 4 4, 289 with 12 8; 8 x 64^3: 53 us with 4 4 4, 61 with
+// 8 8; 2 x 105^3, 7 5 3: 59 us, 63 with last radices up to 8).
+constexpr int XLAST_MAX = 4;
+inline int xfwd_radices(int n, int rmax, int* out) {
+  int rad[FFT_MAX_STAGES];
+  int k = fft_radices(n, rmax, rad), big = rad[0];
+  for (int s = 0; s < k; ++s) out[s] = rad[s];
+  if (k == 1 || rad[k - 1] > XLAST_MAX) out[k++] = 1;
+  for (int r = XLAST_MAX; r >= 2; --r) {
+    if (n % r || n == r) continue;
+    const int q = fft_radices(n / r, rmax, rad) + 1;
+    if (q > k || (q == k && rad[0] >= big)) continue;
+    for (int s = 0; s < q - 1; ++s) out[s] = rad[s];
+    out[q - 1] = r;
+    k = q;
+    big = rad[0];
+  }
+  return k;
 }
 
 // Fill plan p of length n from its radix sequence (stage block lengths and

@@ -644,10 +644,19 @@ template <typename T>
 HD void x_last_split(const cx<T>* buf, cx<T>* spec, long long Nc, const RowMap& rm, int u0, int nf, int nb, int es,
                      const StagePlan& p, const int* ip, const cx<T>* wz, int tid, int nthr) {
   const int R = p.R[p.nst - 1], M = p.n / R;
-#define OFDFT_RADIX_DO(r) x_last_split_r<T, r>(buf, spec, Nc, rm, u0, nf, nb, es, M, ip, wz, tid, nthr)
-  if (R == 1) OFDFT_RADIX_DO(1);
-  else OFDFT_RADIX_SWITCH(R)
-#undef OFDFT_RADIX_DO
+#define OFDFT_LAST_CASE(r)                                                               \
+  case r:                                                                                \
+    x_last_split_r<T, r>(buf, spec, Nc, rm, u0, nf, nb, es, M, ip, wz, tid, nthr); \
+    break;
+  static_assert(XLAST_MAX == 4, "the radices below");
+  switch (R) {
+    OFDFT_LAST_CASE(1)
+    OFDFT_LAST_CASE(2)
+    OFDFT_LAST_CASE(3)
+    OFDFT_LAST_CASE(4)
+    default: break;
+  }
+#undef OFDFT_LAST_CASE
 }
 
 // Sum and difference with one rounding each: never contracted with the
@@ -728,8 +737,10 @@ HD T pow56(T rho, T a, bool& out) {
 // rho^beta, sqrt(rho) and, when alpha != beta, rho^alpha; WGC: rho, sqrt(rho),
 // then for x = alpha and x = beta: rho^x, theta rho^x, theta^2 rho^x / 2 with
 // theta = rho - rho*), with each power computed once per point: put(f, v) for
-// every field.
-template <typename T, int KS, int NP, class Put>
+// every field.  POW56: the WT functional with both exponents 5/6 (its fall-back
+// power is a call).  Every index is a constant: arrays indexed in a loop go to
+// local memory.
+template <typename T, int KS, bool POW56, int NP, class Put>
 HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Put put) {
   T rho[NP], sq[NP], v[NP];
 #pragma unroll
@@ -740,23 +751,27 @@ HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Pu
   put(0, rho);
   put(KS == KS_WT ? 2 : 1, sq);
   if constexpr (KS == KS_WT) {
-    bool slow = !fp.pow56;
-    if (fp.pow56) {
+    if constexpr (POW56) {
+      bool slow = false;
 #pragma unroll
       for (int k = 0; k < NP; ++k) v[k] = pow56(rho[k], sq[k], slow);
-    }
-    if (slow) {
-#pragma unroll 1
+      if (slow) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) v[k] = m_pow_call(rho[k], fp.beta);
+      }
+      put(1, v);
+    } else {
+#pragma unroll
       for (int k = 0; k < NP; ++k) v[k] = m_pow(rho[k], fp.beta);
-    }
-    put(1, v);
-    if (nf > 3) {
-#pragma unroll 1
-      for (int k = 0; k < NP; ++k) v[k] = m_pow(rho[k], fp.alpha);
-      put(3, v);
+      put(1, v);
+      if (nf > 3) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) v[k] = m_pow(rho[k], fp.alpha);
+        put(3, v);
+      }
     }
   } else {
-#pragma unroll 1
+#pragma unroll
     for (int h = 0; h < 2; ++h) {
 #pragma unroll
       for (int k = 0; k < NP; ++k) v[k] = m_pow(rho[k], h == 0 ? fp.alpha : fp.beta);
@@ -819,32 +834,62 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
       }
     }
   };
-  for (int f0 = 0; f0 < (ev == EV_ION ? nf : 1); ++f0) {
-    const T* __restrict__ A = ev == EV_ION ? (const T*)s.buf[B_PHI + f0] : in.A;
-#pragma unroll 2
-    for (int w = tid; w < nb * n1; w += nthr) {
-      const int b = magic_div32(w, mn1), i = w - b * n1;
-      const bool has1 = rm.has1(u0 + b);
-      const int i0 = rm.row(u0 + b, 0) * n1 + i, i1 = has1 ? i0 + n1 : i0;
-      cx<T>* d = buf + i * es + b;
+  if (!setup && (KS == KS_WGC || !fp.pow56)) {
+    // General powers: a work item is one row of a pair (and its partner n3/2
+    // further), so that twice as many threads each compute half as many powers
+    // one after the other (8 x 64^3, unequal exponents: 118 us of the pass with
+    // the pair as the item, its powers in loops over local memory, and a last
+    // stage of radix 8; 89 us so).  Consecutive threads take the two rows of a
+    // pair: their fields are the two parts of one complex value.
+    for (int w = tid; w < 2 * nb * n1; w += nthr) {
+      const int p = w & 1, b = magic_div32(w >> 1, mn1), i = (w >> 1) - b * n1;
+      const bool has = p == 0 || rm.has1(u0 + b);
+      const int i0 = (rm.row(u0 + b, 0) + (has ? p : 0)) * n1 + i;
+      T* d = (T*)(buf + i * es + b) + p;
       if (zs == 1) {
-        const int idx[2] = {i0, i1};
-        T x[2];
-        inputs(Count<2>(), A, idx, x);
-        auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], has1 ? v[1] : T(0)); };
-        if (setup) put(f0, x);
-        else point_fields<T, KS, 2>(fp, in.rho_mode, nf, x, put);
+        const int idx[1] = {i0};
+        T x[1];
+        inputs(Count<1>(), in.A, idx, x);
+        point_fields<T, KS, false, 1>(fp, in.rho_mode, nf, x,
+                                      [&](int f, const T* v) { d[2 * (f * nc)] = has ? v[0] : T(0); });
       } else {
-        const int hs = rm.half * n1;
-        const int idx[4] = {i0, i1, i0 + hs, i1 + hs};
-        T x[4];
-        inputs(Count<4>(), A, idx, x);
-        auto put = [&](int f, const T* v) {
-          d[f * nc] = mk<T>(add_rn(v[0], v[2]), has1 ? add_rn(v[1], v[3]) : T(0));
-          d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), has1 ? add_rn(v[1], -v[3]) : T(0));
-        };
-        if (setup) put(f0, x);
-        else point_fields<T, KS, 4>(fp, in.rho_mode, nf, x, put);
+        const int idx[2] = {i0, i0 + rm.half * n1};
+        T x[2];
+        inputs(Count<2>(), in.A, idx, x);
+        point_fields<T, KS, false, 2>(fp, in.rho_mode, nf, x, [&](int f, const T* v) {
+          d[2 * (f * nc)] = has ? add_rn(v[0], v[1]) : T(0);
+          d[2 * (f * nc + nb)] = has ? add_rn(v[0], -v[1]) : T(0);
+        });
+      }
+    }
+  } else {
+    for (int f0 = 0; f0 < (ev == EV_ION ? nf : 1); ++f0) {
+      const T* __restrict__ A = ev == EV_ION ? (const T*)s.buf[B_PHI + f0] : in.A;
+#pragma unroll 2
+      for (int w = tid; w < nb * n1; w += nthr) {
+        const int b = magic_div32(w, mn1), i = w - b * n1;
+        const bool has1 = rm.has1(u0 + b);
+        const int i0 = rm.row(u0 + b, 0) * n1 + i, i1 = has1 ? i0 + n1 : i0;
+        cx<T>* d = buf + i * es + b;
+        if (zs == 1) {
+          const int idx[2] = {i0, i1};
+          T x[2];
+          inputs(Count<2>(), A, idx, x);
+          auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], has1 ? v[1] : T(0)); };
+          if (setup) put(f0, x);
+          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 2>(fp, in.rho_mode, nf, x, put);
+        } else {
+          const int hs = rm.half * n1;
+          const int idx[4] = {i0, i1, i0 + hs, i1 + hs};
+          T x[4];
+          inputs(Count<4>(), A, idx, x);
+          auto put = [&](int f, const T* v) {
+            d[f * nc] = mk<T>(add_rn(v[0], v[2]), has1 ? add_rn(v[1], v[3]) : T(0));
+            d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), has1 ? add_rn(v[1], -v[3]) : T(0));
+          };
+          if (setup) put(f0, x);
+          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 4>(fp, in.rho_mode, nf, x, put);
+        }
       }
     }
   }
