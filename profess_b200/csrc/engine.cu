@@ -70,28 +70,14 @@ static int d2h(void* h, const void* d, size_t n) { return cuda_check(cudaMemcpy(
 static int dsync() { return cuda_check(cudaDeviceSynchronize(), "synchronize"); }
 #endif
 
-// Launch shape of a slot's passes: row pairs per x-forward task (*rp1) and
-// per x-inverse task (s.rp), 32 at most, whose transform buffers (every field
-// or ion species) fit the KB of shared memory below, and the tiles of the
-// split y/z path: z columns per y-pass task (*ty: columns of n2 values at an
-// odd row pitch) and y columns per z-pass task (*tz: a group of gmax fields of
-// zh values each), each in about 48 KB, at least 32 and 16 columns when n
-// allows (160 x 160 x 256 WGC FP64: 16 columns of a z task 340 us, 32 570).
-// Cells too small for 148 tasks of that size still take 24 row pairs (16 x
-// 32^3 FP64: 12 + 18 us; every task is a fixed chain of latencies, so more and
-// smaller ones cost more than they spread).  s needs n1..n3, k1, nf, kinetic
-// and the plans; csz is the size of one complex value.
-//
-// The FP64 x passes live off resident warps: three 256-thread blocks (16 x
-// 96^3: forward 248 us with 74-78 KB and radices up to 8, 276 with radices up
-// to 12; inverse 368-370 with 56-74 KB; with two blocks of 110 KB at 128
-// registers 303 and 457).
-#ifndef OFDFT_XF_KB64
-#define OFDFT_XF_KB64 78
-#endif
-#ifndef OFDFT_XI_KB64
-#define OFDFT_XI_KB64 56
-#endif
+// Launch shape of a slot's passes: row pairs per x-inverse task (s.rp), at most
+// so many per x-forward task (*rp1; a launch may take smaller ones, see
+// xfwd_points), 32 at most, and the tiles of the split y/z path: z columns per
+// y-pass task (*ty: columns of n2 values at an odd row pitch) and y columns per
+// z-pass task (*tz: a group of gmax fields of zh values each), each in about 48
+// KB, at least 32 and 16 columns when n allows (160 x 160 x 256 WGC FP64: 16
+// columns of a z task 340 us, 32 570).  s needs n1..n3, k1, nf, kinetic and the
+// plans; csz is the size of one complex value.
 #ifndef OFDFT_X_THREADS
 #define OFDFT_X_THREADS 256
 #endif
@@ -119,16 +105,91 @@ static size_t xi_smem(const SlotDev& s, int nfb, int rp, size_t esz) {
 #endif
   return xinv_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
 }
+
+constexpr int X_MAX_RP = 32;  // most row pairs of an x task
+
+// Model time of a launch of FP64 x-forward blocks, in points of one field's row
+// pairs: whole waves of resident blocks (three an SM by registers, fewer by
+// shared memory), each a fixed chain of latencies worth about 1000 points and
+// the block's own points (three fields), which cost less where fewer blocks
+// share an SM.  (Fitted to 33 shapes from 24^3 to 160 x 160 x 256.)
+static double xfwd_cost(long long tasks, double points, size_t smem, int sms) {
+  const int o = std::max(1, std::min(3, (int)(233472 / (smem + 1024))));
+  static const double share[4] = {0.0, 0.65, 0.85, 1.0};
+  const long long waves = (tasks + (long long)o * sms - 1) / ((long long)o * sms);
+  return (double)waves * (1000.0 + points * share[o]);
+}
+
+// Row pairs per x-inverse task of an FP64 slot: as many as fit the shared
+// memory below.  The order of its sums follows the tasks, so the size can not
+// depend on what else is launched, as the x-forward pass's does.  With the row
+// split 66 KB and 24 row pairs, more where a cell has work for 148 tasks of
+// more (every task is a fixed chain of latencies; but larger tasks than that
+// leave the spilled registers no L1: 16 x 96^3 354 us with 12, 368 with 14; 3 x
+// 72^3 30 us with 18, 42 with 14); without it 72 KB and 32 (12 x 45^3: 29 us, 41
+// with 24; 6 x 75^3: 71 us with 20, 79 with 15); WGC 68 KB (4 x 64^3 80 us with
+// 8, 91 with 6).
+static int xinv_row_pairs(const SlotDev& s) {
+  const int nrp = (s.n2 * s.n3 + 1) / 2;
+  const size_t kb = s.kinetic == KIN_WGC ? 68 : s.zs == 1 ? 72 : 66;
+  int r = s.zs == 1 ? X_MAX_RP : std::max(24, std::min(X_MAX_RP, (nrp + 147) / 148));
+  while (r > s.zs && xi_smem(s, s.nf, r, 8) > kb * 1024) r--;
+  return r;
+}
+
+// An x-forward launch's cells.  The task size changes no result (each column is
+// transformed by itself), so a launch takes the points a task whose model time
+// for all its cells is least.  16 x 96^3 FP64: 258 us with 12 row pairs for every
+// batch, 227 with the 16 of this rule; 8 x 64^3 52 -> 38; one 108^3 40 -> 24.
+struct XfwdCell {
+  int n1, zs, nunits, nf, rp_max;
+  // units of a task of about that many points
+  int units(double points) const {
+    return std::max(1, std::min(rp_max / zs, (int)(points / ((double)zs * n1))));
+  }
+};
+static double xfwd_points(const XfwdCell* cells, int n, int sms) {
+  // candidates: the sizes of the cell with the most work
+  int big = 0;
+  auto work = [](const XfwdCell& c) { return (double)c.nunits * c.zs * c.n1 * c.nf; };
+  for (int k = 1; k < n; ++k)
+    if (work(cells[k]) > work(cells[big])) big = k;
+  const XfwdCell& b = cells[big];
+  double pick = 0.0, least = 0.0;
+  for (int u = 1; u <= std::max(1, b.rp_max / b.zs); ++u) {
+    const double points = (double)u * b.zs * b.n1;
+    long long tasks = 0;
+    size_t sm = 0;
+    double most = 0.0;
+    for (int k = 0; k < n; ++k) {
+      const XfwdCell& c = cells[k];
+      const int uc = c.units(points);
+      tasks += (c.nunits + uc - 1) / uc;
+      sm = std::max(sm, xfwd_smem(c.n1, c.nf, uc * c.zs, 8));
+      most = std::max(most, (double)uc * c.zs * c.n1 * c.nf / 3.0);
+    }
+    const double t = xfwd_cost(tasks, most, sm, sms);
+    if (u == 1 || t < least) {
+      least = t;
+      pick = points;
+    }
+  }
+  return pick;
+}
+
 static void launch_shape(SlotDev& s, size_t csz, int nfx, int* rp1, int* ty, int* tz) {
   const size_t esz = csz / 2;
   const bool f32 = csz == 8;
-  const int nrp = (s.n2 * s.n3 + 1) / 2;
-  const int most = f32 ? std::max(1, std::min(32, 2048 / s.n1)) : std::max(24, std::min(32, (nrp + 147) / 148));
-  const size_t fkb = (f32 ? 48 : OFDFT_XF_KB64) * 1024, ikb = (f32 ? 48 : OFDFT_XI_KB64) * 1024;
+  const int most = f32 ? std::max(1, std::min(X_MAX_RP, 2048 / s.n1)) : X_MAX_RP;
+  const size_t fkb = (f32 ? 48 : 160) * 1024, ikb = 48 * 1024;
   *rp1 = most;
   while (*rp1 > s.zs && xf_smem(s, nfx, *rp1, esz) > fkb) (*rp1)--;
-  s.rp = most;
-  while (s.rp > s.zs && xi_smem(s, s.nf, s.rp, esz) > ikb) s.rp--;
+  if (f32) {
+    s.rp = most;
+    while (s.rp > s.zs && xi_smem(s, s.nf, s.rp, esz) > ikb) s.rp--;
+  } else {
+    s.rp = xinv_row_pairs(s);
+  }
   const int gmax = s.kinetic == KIN_WGC ? 3 : 1;
   const size_t ycol = (size_t)(s.n2 | 1) * csz, zcol = (size_t)gmax * s.zh * csz;
   *ty = (int)std::max<size_t>(1, std::min<size_t>(s.n3, std::max<size_t>(48 * 1024 / ycol, 32)));
@@ -153,11 +214,50 @@ constexpr size_t YZ_SMEM_MAX = 226 * 1024;
 // blocks beat one 512-thread block on 84-99 KB plane sets (WT 72^3 FP64,
 // 108^3 FP32, WGC 64^3 FP32: 9-11 % faster evaluations).
 constexpr size_t YZ_SMEM_SMALL = 112 * 1024;
-// Threads of a block of the small class: about one per butterfly of radix 8
-// (a stage's work items), 64 to 192.  16 x 32^3 FP64: 30 us with 256 threads,
-// 19 with 128; 16 x 96^3 FP64: 345 with 256, 333 with 192, 370 with 128.
-static int yz_threads(const SlotDev& s) {
-  return std::max(64, std::min(192, (s.n2 * s.zh / 8 + 31) / 32 * 32));
+// Threads of the blocks of an FP64 launch of the small class.  They change no
+// result, so a launch takes the number whose model time is least: whole waves
+// of resident blocks (by shared memory, and 768 threads an SM by registers),
+// each a fixed latency, the rounds of butterflies over the block's threads, and
+// the points of an SM's resident blocks (in us: 4, 0.55 and 1.23 a thousand,
+// fitted to launches of 1 to 64 cells of 20^3 to 108^3).  Half of a WGC cell's
+// tasks hold three planes, half one: their mean, and no whole waves, since the
+// short ones fill the last.  The smaller number unless a larger one gains 3 %
+// (160 and 224 threads, an odd number of warps, lose up to a quarter).  With one number per shape,
+// 64 to 192 by points, before: 12 x 45^3 42 us, 33 so; 8 x 64^3 58, 51; 12 x 48^3 49,
+// 39; 6 x 75^3 112, 106; one 108^3 59, 54; 4 x 64^3 WGC 124, 113; 16 x 32^3 and 16 x
+// 96^3 as before (14 and 330; 30 and 336 with 256).
+struct YzCell {
+  const SlotDev* s;
+  long long tasks;
+};
+static int yz_threads(const YzCell* cells, int n, size_t smem, int sms) {
+  static const int threads[5] = {64, 96, 128, 192, 256};
+  long long tasks = 0;
+  for (int k = 0; k < n; ++k) tasks += cells[k].tasks;
+  int pick = threads[0];
+  double least = 0.0;
+  for (int nt : threads) {
+    const int o = std::max(1, std::min((int)(233472 / (smem + 1024)), 768 / nt));
+    double rounds = 0.0, points = 0.0;  // means of a task
+    for (int k = 0; k < n; ++k) {
+      const SlotDev& s = *cells[k].s;
+      const int pts = s.n2 * s.zh * (s.kinetic == KIN_WGC ? 2 : 1);
+      int r = 0;
+      for (const StagePlan* p : {&s.qy, &s.qzh})
+        for (int st = 0; st < p->nst; ++st) r += (pts / p->R[st] + nt - 1) / nt;
+      rounds += (double)r * (double)cells[k].tasks / (double)tasks;
+      points += (double)pts * (double)cells[k].tasks / (double)tasks;
+    }
+    double waves = std::max(1.0, (double)tasks / ((double)o * sms));
+    if (cells[0].s->kinetic == KIN_WT) waves = std::ceil(waves);
+    const double resident = (double)std::min<long long>(o, (tasks + sms - 1) / sms);
+    const double t = waves * (4.0 + 0.55 * rounds + 1.23e-3 * points * resident);
+    if (nt == threads[0] || t < 0.97 * least) {
+      least = t;
+      pick = nt;
+    }
+  }
+  return pick;
 }
 
 // ------------------------------------------------------------ FFT plans
@@ -368,7 +468,7 @@ struct HostSlot {
   SlotDev sd;
   std::vector<std::pair<void*, size_t>> allocs;  // device blocks and their sizes
   int nunits = 0;               // units of the x passes: pairs of rows, with the row split two pairs each
-  int rp1 = 1;                  // row pairs per x-forward task
+  int rp1 = 1;                  // row pairs per x-forward task (FP64: at most)
   int ty = 1, tz = 1;           // z columns per y-pass task and y columns per z-pass task (split path)
   int xcap = 0;                 // radix cap of the x-axis plan (0: the default)
   int yzt = 0;                  // threads of the fused y-z pass (0: by plane size)
@@ -1882,6 +1982,10 @@ struct Engine {
     return !h.setup_pass && yz_smem_slot(h.sd, 2 * elem_size(h.prec)) <= YZ_SMEM_MAX;
   }
 
+  static XfwdCell xfwd_cell(const HostSlot& h) {
+    return {h.sd.n1, h.sd.zs, h.nunits, std::max(h.sd.nf, h.sd.ion.nspec), std::max(h.rp1, h.sd.zs)};
+  }
+
   int build_lists() {
     for (int p = 0; p < 2; ++p)
       for (int k = 0; k < NPASS; ++k) {
@@ -1889,6 +1993,13 @@ struct Engine {
         lists[p][k].smem = 0;
         lists[p][k].nthr = 0;
       }
+    std::vector<XfwdCell> cells[2];  // the FP64 cells of the x-forward launches (WT, WGC)
+    for (int i = 0; i < cap; ++i)
+      if (slots[i].used && slots[i].running && slots[i].prec == OFDFT_FP64)
+        cells[slots[i].sd.kinetic == KIN_WGC].push_back(xfwd_cell(slots[i]));
+    std::vector<YzCell> yz_cells[2];  // those of its y-z launches of the small class, the block size not pinned
+    double points[2];
+    for (int w = 0; w < 2; ++w) points[w] = cells[w].empty() ? 0.0 : xfwd_points(cells[w].data(), (int)cells[w].size(), num_sms);
     for (int i = 0; i < cap; ++i) {
       HostSlot& h = slots[i];
       if (!h.used || !h.running) continue;
@@ -1900,10 +2011,10 @@ struct Engine {
       L[P_VEC].smem = std::max(L[P_VEC].smem, (size_t)(NCH * 33 * sizeof(double) + 16));
       const bool wgc = s.kinetic == KIN_WGC;
       const int px1 = wgc ? P_X1G : P_X1, pz3 = wgc ? P_Z3G : P_Z3, px5 = wgc ? P_X5G : P_X5;
-      const int u1 = x_units(s, h.rp1), u5 = x_units(s, s.rp);
+      const int u1 = h.prec == OFDFT_FP64 ? xfwd_cell(h).units(points[wgc]) : h.rp1, u5 = x_units(s, s.rp);
       for (int r = 0; r < h.nunits; r += u1) L[px1].h.push_back({i, 0, r, std::min(u1, h.nunits - r)});
       L[px1].nthr = X_THREADS;
-      L[px1].smem = std::max(L[px1].smem, xf_smem(s, std::max(s.nf, s.ion.nspec), h.rp1, cs / 2));
+      L[px1].smem = std::max(L[px1].smem, xf_smem(s, std::max(s.nf, s.ion.nspec), u1 * s.zs, cs / 2));
       if (uses_yz(h)) {  // fused y-z pass: one task per (field, kx)
         const size_t sm = yz_smem_slot(s, cs);
         const bool big = h.yzt == 256 ? false : h.yzt == 512 ? true : sm > YZ_SMEM_SMALL;
@@ -1913,8 +2024,9 @@ struct Engine {
         for (int g = s.ngroups - 1; g >= 0; --g)
           for (int kx = 0; kx < s.k1; ++kx)
             for (int hf = 0; hf < s.zs; ++hf) L[pyz].h.push_back({i, g, kx, hf});
-        L[pyz].nthr = big ? 512 : std::max(h.yzt ? h.yzt : h.prec == OFDFT_FP32 ? 256 : yz_threads(s), L[pyz].nthr);
         L[pyz].smem = std::max(L[pyz].smem, sm);
+        if (big || h.yzt || h.prec == OFDFT_FP32) L[pyz].nthr = big ? 512 : 256;
+        else yz_cells[wgc].push_back({&s, (long long)s.ngroups * s.k1 * s.zs});
       } else {  // split path: y forward, z with the operator, y inverse
         for (int pass : {P_Y2, P_Y4}) {
           for (int f = 0; f < s.nf; ++f)
@@ -1939,6 +2051,10 @@ struct Engine {
       L[P_CTL].smem = 0;
       L[px5].nthr = X_THREADS;
       L[px5].smem = std::max(L[px5].smem, xi_smem(s, std::max(s.nf, s.ion.nspec), s.rp, cs / 2));
+    }
+    for (int w = 0; w < 2; ++w) {
+      LaunchList& l = lists[OFDFT_FP64][w ? P_YZG : P_YZ];
+      if (!yz_cells[w].empty() && !l.nthr) l.nthr = yz_threads(yz_cells[w].data(), (int)yz_cells[w].size(), l.smem, num_sms);
     }
 #if defined(OFDFT_EMU)
     for (int p = 0; p < 2; ++p)
@@ -2665,6 +2781,7 @@ constexpr size_t SCRATCH_BYTES = size_t(12) << 20;  // 12 MiB
 constexpr long long MAX_POINTS = 262144;             // 64^3 grid points
 constexpr int MAX_DIM = 128;
 constexpr int MAX_TASKS = 12288;
+constexpr int B200_SMS = 148;
 constexpr int MAX_DEVICES = 128;
 static __device__ __align__(256) unsigned char g_scratch[SCRATCH_BYTES];
 static void* g_addr[MAX_DEVICES];  // device address of g_scratch per device ordinal
@@ -2783,7 +2900,8 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   const int nrows = s.n2 * s.n3, nrp = (nrows / s.zs + 1) / 2;  // units
   int rp1 = 1, ty = 1, tz = 1;
   launch_shape(s, cs, s.nf, &rp1, &ty, &tz);  // the engine's own launch shape
-  const int u1 = x_units(s, rp1), u5 = x_units(s, s.rp);
+  const XfwdCell cell{s.n1, s.zs, nrp, s.nf, rp1};
+  const int u1 = cell.units(xfwd_points(&cell, 1, B200_SMS)), u5 = x_units(s, s.rp);
   s.ntask[K_X5] = (nrp + u5 - 1) / u5;
   s.buf[B_PHI] = (void*)rho;         // the input density (read only in EV_RHO mode)
   s.buf[B_W0] = (void*)potential;    // the output potential
@@ -2791,7 +2909,8 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   // the engine's passes: the fused y-z pass when the plane fits, else the split path
   const size_t yzsm = yz_smem(s, cs);
   const bool fused = yzsm <= YZ_SMEM_MAX;
-  const int yzthr = yzsm <= YZ_SMEM_SMALL ? yz_threads(s) : 512;
+  const YzCell yz{&s, (long long)s.ngroups * s.k1 * s.zs};
+  const int yzthr = yzsm <= YZ_SMEM_SMALL ? yz_threads(&yz, 1, yzsm, B200_SMS) : 512;
   // task lists, packed one pass after the other: x forward, y forward (or
   // y-z), z, y inverse, x inverse, controller
   int nt[6] = {0, 0, 0, 0, 0, 0}, ntot = 0;
