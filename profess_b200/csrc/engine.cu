@@ -1370,23 +1370,31 @@ struct Engine {
 #else
   void* d_io = nullptr;
   size_t io_bytes = 0;
+  // It grows in steps - powers of two from 256 KiB to 64 MiB, then multiples of
+  // that - since a step costs a cudaFree, which waits for the device, and a
+  // cudaMalloc; to the exact size where memory is short.
   int io_scratch(size_t bytes, void** p) {
     if (io_bytes < bytes) {
+      constexpr size_t least = size_t(1) << 18, most = size_t(64) << 20;
+      size_t n = least;
+      while (n < bytes && n < most) n *= 2;
+      if (n < bytes) n = (bytes + most - 1) / most * most;
       dfree(d_io);
       d_io = nullptr;
       io_bytes = 0;
-      int rc = cuda_check(cudaMalloc(&d_io, bytes), "cudaMalloc");
+      int rc = cuda_check(cudaMalloc(&d_io, n), "cudaMalloc");
       if (rc == OFDFT_ENOMEM) {
         cudaGetLastError();  // must not show up as a later launch error
         pool_flush();
-        rc = cuda_check(cudaMalloc(&d_io, bytes), "cudaMalloc");
+        n = bytes;
+        rc = cuda_check(cudaMalloc(&d_io, n), "cudaMalloc");
       }
       if (rc) {
         cudaGetLastError();
         d_io = nullptr;
         return rc;
       }
-      io_bytes = bytes;
+      io_bytes = n;
     }
     *p = d_io;
     return OFDFT_OK;
@@ -1547,11 +1555,13 @@ struct Engine {
     return OFDFT_OK;
 #else
     // one scratch array (the engine's transfer scratch): phases, S(G), the
-    // outputs, then frac and z (one copy up, one copy down)
+    // outputs, then frac and z (one copy up, one copy down); its size does not
+    // depend on whether forces are wanted
     std::vector<double> in(h.frac);
     in.insert(in.end(), h.zion.begin(), h.zion.end());
     char* scratch = nullptr;
-    int rc = io_scratch(sizeof(cx<double>) * (nph + nsf) + sizeof(double) * (out.size() + in.size()), (void**)&scratch);
+    int rc = io_scratch(sizeof(cx<double>) * (nph + nsf) +
+                            sizeof(double) * ((size_t)NOUT * nsum + 3 * (size_t)nion + in.size()), (void**)&scratch);
     if (rc) return rc;
     cx<double>* dtab = (cx<double>*)scratch;
     cx<double>* dsf = dtab + nph;
