@@ -28,8 +28,11 @@ EMU_PATH = os.path.join(EMU_DIR, "libprofess_b200_emu.so")
 # engine.cu and, one unit per pass and precision, the pass kernels
 PASS_UNITS = ["pass_%s_%s.cu" % (p, t) for t in ("f64", "f32") for p in ("yzg", "yz", "split", "xfwd", "xinv")]
 SOURCES = ["engine.cu"] + PASS_UNITS
-HEADERS = ["kernels.cuh", "cx.cuh", "fft.cuh", "dcsrch.cuh", "slot.cuh", "ntn_ctl.cuh", "passes.cuh", "setup.cuh", "ewald.cuh", "stress.cuh"] + [
-    "f32/%s.cuh" % h for h in ("kernels", "cx", "fft", "dcsrch", "slot", "ntn_ctl", "passes")]
+HEADERS = ["%s.cuh" % h for h in ("kernels", "cx", "dft", "fft", "dcsrch", "slot", "ntn_ctl", "pass_common", "passes", "setup",
+                                  "ewald", "stress")] + [
+    "f32/%s.cuh" % h for h in ("kernels", "instantiate", "async", "fft", "shape", "passes")]
+# the host emulation: engine.cu takes the FP64 block functions from the headers
+EMU_SOURCES = ["engine.cu"] + [u for u in PASS_UNITS if u.endswith("_f32.cu")]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
@@ -88,7 +91,7 @@ def build_emu(force: bool = False) -> str:
         return EMU_PATH
     os.makedirs(EMU_DIR, exist_ok=True)
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fopenmp", "-DOFDFT_EMU", "-x", "c++",
-           "-I", INCLUDE, "-I", CSRC, os.path.join(CSRC, "engine.cu"), "-o", EMU_PATH]
+           "-I", INCLUDE, "-I", CSRC] + [os.path.join(CSRC, s) for s in EMU_SOURCES] + ["-o", EMU_PATH]
     subprocess.run(cmd, check=True)
     return EMU_PATH
 

@@ -48,29 +48,6 @@ template <typename T> HD cx<T> mul_i(cx<T> a, int dir) {
   return dir > 0 ? mk<T>(-a.y, a.x) : mk<T>(a.y, -a.x);
 }
 
-// Two adjacent complex values: one 16-byte access in FP32 (p must then be
-// 16-byte aligned), two in FP64.
-template <typename T> struct Cx2 { cx<T> a, b; };
-template <typename T> HD Cx2<T> ld_cx2(const cx<T>* p) {
-#if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) {
-    const float4 q = *(const float4*)p;
-    return Cx2<T>{mk<T>(q.x, q.y), mk<T>(q.z, q.w)};
-  }
-#endif
-  return Cx2<T>{p[0], p[1]};
-}
-template <typename T> HD void st_cx2(cx<T>* p, cx<T> a, cx<T> b) {
-#if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) {
-    *(float4*)p = make_float4(a.x, a.y, b.x, b.y);
-    return;
-  }
-#endif
-  p[0] = a;
-  p[1] = b;
-}
-
 // Precision-generic math wrappers (float versions map to the float library calls).
 HD double m_sqrt(double v) { return sqrt(v); }
 HD float m_sqrt(float v) { return sqrtf(v); }
@@ -82,10 +59,8 @@ HD float m_pow(float a, float b) { return powf(a, b); }
 // the common one.
 #if defined(__CUDA_ARCH__)
 __device__ __noinline__ inline double m_pow_call(double a, double b) { return pow(a, b); }
-__device__ __noinline__ inline float m_pow_call(float a, float b) { return powf(a, b); }
 #else
 HD double m_pow_call(double a, double b) { return pow(a, b); }
-HD float m_pow_call(float a, float b) { return powf(a, b); }
 #endif
 HD double m_log(double v) { return log(v); }
 HD float m_log(float v) { return logf(v); }

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "f32/kernels.cuh"
 #include "setup.cuh"
 #include "ewald.cuh"
 #include "stress.cuh"
@@ -84,26 +85,15 @@ static int dsync() { return cuda_check(cudaDeviceSynchronize(), "synchronize"); 
 constexpr int X_THREADS = OFDFT_X_THREADS;  // threads of an x-pass block
 // Units of an x task of rp row pairs (at least one).
 static int x_units(const SlotDev& s, int rp) { return std::max(1, rp / s.zs); }
-// The FP32 passes (f32/) have a shape rule of their own: 256-thread blocks, row
-// pairs whose buffers (forward: and the staged rows of the two inputs) fit 48
-// KB, up to 2048 points.  The host emulation runs the FP64 passes' code.
-static size_t f32_xfwd_smem(int n1, int nfb, int nb, size_t esz) {
-  return align16((size_t)nfb * nb * n1 * 2 * esz) + 2 * align16((size_t)2 * nb * n1 * esz);
-}
-static size_t f32_xinv_smem(int n1, int nfb, int nb, size_t esz) {
-  return align16((size_t)nfb * nb * n1 * 2 * esz) + NCH * 33 * sizeof(double);
-}
+// Shared memory of the x passes with nfb fields (or ion species) and rp row
+// pairs a task.  The FP32 passes have a shape rule of their own: row pairs whose
+// buffers (forward: and the staged rows of the two inputs) fit 48 KB, up to 2048
+// points.
 static size_t xf_smem(const SlotDev& s, int nfb, int rp, size_t esz) {
-#if !defined(OFDFT_EMU)
-  if (esz == 4) return f32_xfwd_smem(s.n1, nfb, rp, esz);
-#endif
-  return xfwd_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
+  return esz == 4 ? f32::xfwd_smem(s.n1, nfb, rp, esz) : xfwd_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
 }
 static size_t xi_smem(const SlotDev& s, int nfb, int rp, size_t esz) {
-#if !defined(OFDFT_EMU)
-  if (esz == 4) return f32_xinv_smem(s.n1, nfb, rp, esz);
-#endif
-  return xinv_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
+  return esz == 4 ? f32::xinv_smem(s.n1, nfb, rp, esz) : xinv_smem(s.n1, nfb, x_units(s, rp) * s.zs, esz);
 }
 
 constexpr int X_MAX_RP = 32;  // most row pairs of an x task
@@ -387,6 +377,46 @@ enum Pass : int { P_VEC = 0, P_X1 = 1, P_Y2 = 2, P_Z3 = 3, P_Y4 = 4, P_X5 = 5, P
                   NPASS = 14 };
 constexpr int VEC_PER_TICK = 2;
 constexpr int VCHUNK = 4096;
+
+// The pass kernels of a precision (in the host emulation, their block functions).
+template <typename T> struct PassKernels {
+  static constexpr bool F64 = sizeof(T) == 8;
+#if defined(OFDFT_EMU)
+#define OFDFT_PASS_BLOCK(name)                                              \
+  template <int KS> static void name(const Args<T>& a, int b, char* sm) {   \
+    if constexpr (F64) ofdft::name<T, KS>(a, b, 0, 1, sm);                  \
+    else f32::name<T, KS>(a, b, 0, 1, sm);                                  \
+  }
+  OFDFT_PASS_BLOCK(xfwd_block)
+  OFDFT_PASS_BLOCK(zpass_block)
+  OFDFT_PASS_BLOCK(yzpass_block)
+  OFDFT_PASS_BLOCK(xinv_block)
+#undef OFDFT_PASS_BLOCK
+  static void ypass_block(const Args<T>& a, int b, char* sm, int dir) {
+    if constexpr (F64) ofdft::ypass_block<T>(a, b, 0, 1, sm, dir);
+    else f32::ypass_block<T>(a, b, 0, 1, sm, dir);
+  }
+#else
+  using Kernel = void (*)(Args<T>);
+#define OFDFT_PASS_KERNEL(name)                  \
+  template <int KS> static Kernel name() {       \
+    if constexpr (F64) return k_##name<T, KS>;   \
+    else return f32::k_##name<T, KS>;            \
+  }
+  OFDFT_PASS_KERNEL(xfwd)
+  OFDFT_PASS_KERNEL(zpass)
+  OFDFT_PASS_KERNEL(xinv)
+#undef OFDFT_PASS_KERNEL
+  template <int NT, int KS> static Kernel yzpass() {
+    if constexpr (F64) return k_yzpass<T, NT, KS>;
+    else return f32::k_yzpass<T, NT, KS>;
+  }
+  static void (*ypass())(Args<T>, int) {
+    if constexpr (F64) return k_ypass<T>;
+    else return f32::k_ypass<T>;
+  }
+#endif
+};
 
 #if !defined(OFDFT_EMU)
 template <typename T> __global__ void __launch_bounds__(256) k_vec(Args<T> a) {
@@ -2128,18 +2158,18 @@ struct Engine {
       run(P_VEC, [](Args<T>& a, int b, char* sm) { vec_block<T>(a, b, 0, 1, sm); });
       run(P_CTL, [](Args<T>& a, int b, char*) { ctl_block(a.slots, a.ctl, a.tasks, K_VEC, b, 0, 1, (char*)ctl_sm); });
     }
-    run(P_X1, [](Args<T>& a, int b, char* sm) { xfwd_block<T, KS_WT>(a, b, 0, 1, sm); });
-    run(P_X1G, [](Args<T>& a, int b, char* sm) { xfwd_block<T, KS_WGC>(a, b, 0, 1, sm); });
-    run(P_Y2, [](Args<T>& a, int b, char* sm) { ypass_block<T>(a, b, 0, 1, sm, -1); });
-    run(P_Z3, [](Args<T>& a, int b, char* sm) { zpass_block<T, KS_WT>(a, b, 0, 1, sm); });
-    run(P_Z3G, [](Args<T>& a, int b, char* sm) { zpass_block<T, KS_WGC>(a, b, 0, 1, sm); });
-    run(P_Y4, [](Args<T>& a, int b, char* sm) { ypass_block<T>(a, b, 0, 1, sm, 1); });
-    run(P_YZ, [](Args<T>& a, int b, char* sm) { yzpass_block<T, KS_WT>(a, b, 0, 1, sm); });
-    run(P_YZB, [](Args<T>& a, int b, char* sm) { yzpass_block<T, KS_WT>(a, b, 0, 1, sm); });
-    run(P_YZG, [](Args<T>& a, int b, char* sm) { yzpass_block<T, KS_WGC>(a, b, 0, 1, sm); });
-    run(P_YZBG, [](Args<T>& a, int b, char* sm) { yzpass_block<T, KS_WGC>(a, b, 0, 1, sm); });
-    run(P_X5, [](Args<T>& a, int b, char* sm) { xinv_block<T, KS_WT>(a, b, 0, 1, sm); });
-    run(P_X5G, [](Args<T>& a, int b, char* sm) { xinv_block<T, KS_WGC>(a, b, 0, 1, sm); });
+    run(P_X1, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template xfwd_block<KS_WT>(a, b, sm); });
+    run(P_X1G, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template xfwd_block<KS_WGC>(a, b, sm); });
+    run(P_Y2, [](Args<T>& a, int b, char* sm) { PassKernels<T>::ypass_block(a, b, sm, -1); });
+    run(P_Z3, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template zpass_block<KS_WT>(a, b, sm); });
+    run(P_Z3G, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template zpass_block<KS_WGC>(a, b, sm); });
+    run(P_Y4, [](Args<T>& a, int b, char* sm) { PassKernels<T>::ypass_block(a, b, sm, 1); });
+    run(P_YZ, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template yzpass_block<KS_WT>(a, b, sm); });
+    run(P_YZB, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template yzpass_block<KS_WT>(a, b, sm); });
+    run(P_YZG, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template yzpass_block<KS_WGC>(a, b, sm); });
+    run(P_YZBG, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template yzpass_block<KS_WGC>(a, b, sm); });
+    run(P_X5, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template xinv_block<KS_WT>(a, b, sm); });
+    run(P_X5G, [](Args<T>& a, int b, char* sm) { PassKernels<T>::template xinv_block<KS_WGC>(a, b, sm); });
     run(P_CTL, [](Args<T>& a, int b, char*) { ctl_block(a.slots, a.ctl, a.tasks, K_X5, b, 0, 1, (char*)ctl_sm); });
     return OFDFT_OK;
   }
@@ -2158,18 +2188,18 @@ struct Engine {
       if ((rc = launch_one<T>(prec, P_VEC, k_vec<T>))) return rc;
       if ((rc = launch_one<T>(prec, P_CTL, k_ctl<T>, (int)K_VEC))) return rc;
     }
-    if ((rc = launch_one<T>(prec, P_X1, k_xfwd<T, KS_WT>))) return rc;
-    if ((rc = launch_one<T>(prec, P_X1G, k_xfwd<T, KS_WGC>))) return rc;
-    if ((rc = launch_one<T>(prec, P_YZ, k_yzpass<T, 256, KS_WT>))) return rc;
-    if ((rc = launch_one<T>(prec, P_YZB, k_yzpass<T, 512, KS_WT>))) return rc;
-    if ((rc = launch_one<T>(prec, P_YZG, k_yzpass<T, 256, KS_WGC>))) return rc;
-    if ((rc = launch_one<T>(prec, P_YZBG, k_yzpass<T, 512, KS_WGC>))) return rc;
-    if ((rc = launch_one<T>(prec, P_Y2, k_ypass<T>, -1))) return rc;
-    if ((rc = launch_one<T>(prec, P_Z3, k_zpass<T, KS_WT>))) return rc;
-    if ((rc = launch_one<T>(prec, P_Z3G, k_zpass<T, KS_WGC>))) return rc;
-    if ((rc = launch_one<T>(prec, P_Y4, k_ypass<T>, 1))) return rc;
-    if ((rc = launch_one<T>(prec, P_X5, k_xinv<T, KS_WT>))) return rc;
-    if ((rc = launch_one<T>(prec, P_X5G, k_xinv<T, KS_WGC>))) return rc;
+    if ((rc = launch_one<T>(prec, P_X1, PassKernels<T>::template xfwd<KS_WT>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_X1G, PassKernels<T>::template xfwd<KS_WGC>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_YZ, PassKernels<T>::template yzpass<256, KS_WT>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_YZB, PassKernels<T>::template yzpass<512, KS_WT>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_YZG, PassKernels<T>::template yzpass<256, KS_WGC>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_YZBG, PassKernels<T>::template yzpass<512, KS_WGC>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_Y2, PassKernels<T>::ypass(), -1))) return rc;
+    if ((rc = launch_one<T>(prec, P_Z3, PassKernels<T>::template zpass<KS_WT>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_Z3G, PassKernels<T>::template zpass<KS_WGC>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_Y4, PassKernels<T>::ypass(), 1))) return rc;
+    if ((rc = launch_one<T>(prec, P_X5, PassKernels<T>::template xinv<KS_WT>()))) return rc;
+    if ((rc = launch_one<T>(prec, P_X5G, PassKernels<T>::template xinv<KS_WGC>()))) return rc;
     return launch_one<T>(prec, P_CTL, k_ctl<T>, (int)K_X5);
   }
 #endif
@@ -2198,17 +2228,17 @@ struct Engine {
     };
     load(k_vec<T>);
     load(k_ctl<T>);
-    load(k_xfwd<T, KS_WT>);
-    load(k_xfwd<T, KS_WGC>);
-    load(k_ypass<T>);
-    load(k_zpass<T, KS_WT>);
-    load(k_zpass<T, KS_WGC>);
-    load(k_yzpass<T, 256, KS_WT>);
-    load(k_yzpass<T, 512, KS_WT>);
-    load(k_yzpass<T, 256, KS_WGC>);
-    load(k_yzpass<T, 512, KS_WGC>);
-    load(k_xinv<T, KS_WT>);
-    load(k_xinv<T, KS_WGC>);
+    load(PassKernels<T>::template xfwd<KS_WT>());
+    load(PassKernels<T>::template xfwd<KS_WGC>());
+    load(PassKernels<T>::ypass());
+    load(PassKernels<T>::template zpass<KS_WT>());
+    load(PassKernels<T>::template zpass<KS_WGC>());
+    load(PassKernels<T>::template yzpass<256, KS_WT>());
+    load(PassKernels<T>::template yzpass<512, KS_WT>());
+    load(PassKernels<T>::template yzpass<256, KS_WGC>());
+    load(PassKernels<T>::template yzpass<512, KS_WGC>());
+    load(PassKernels<T>::template xinv<KS_WT>());
+    load(PassKernels<T>::template xinv<KS_WGC>());
     load(k_permute_kernel<T>);
     load(k_unpermute_kernel<T>);
     load(k_fill_kernel<T>);
@@ -2246,17 +2276,17 @@ struct Engine {
                         "cudaFuncSetAttribute");
     };
     if ((rc = attr(k_vec<T>, P_VEC))) return rc;
-    if ((rc = attr(k_xfwd<T, KS_WT>, P_X1))) return rc;
-    if ((rc = attr(k_xfwd<T, KS_WGC>, P_X1G))) return rc;
-    if ((rc = attr(k_zpass<T, KS_WGC>, P_Z3G))) return rc;
-    if ((rc = attr(k_xinv<T, KS_WGC>, P_X5G))) return rc;
-    if ((rc = attr(k_ypass<T>, lists[prec][P_Y2].smem >= lists[prec][P_Y4].smem ? P_Y2 : P_Y4))) return rc;
-    if ((rc = attr(k_yzpass<T, 256, KS_WT>, P_YZ))) return rc;
-    if ((rc = attr(k_yzpass<T, 512, KS_WT>, P_YZB))) return rc;
-    if ((rc = attr(k_yzpass<T, 256, KS_WGC>, P_YZG))) return rc;
-    if ((rc = attr(k_yzpass<T, 512, KS_WGC>, P_YZBG))) return rc;
-    if ((rc = attr(k_zpass<T, KS_WT>, P_Z3))) return rc;
-    return attr(k_xinv<T, KS_WT>, P_X5);
+    if ((rc = attr(PassKernels<T>::template xfwd<KS_WT>(), P_X1))) return rc;
+    if ((rc = attr(PassKernels<T>::template xfwd<KS_WGC>(), P_X1G))) return rc;
+    if ((rc = attr(PassKernels<T>::template zpass<KS_WGC>(), P_Z3G))) return rc;
+    if ((rc = attr(PassKernels<T>::template xinv<KS_WGC>(), P_X5G))) return rc;
+    if ((rc = attr(PassKernels<T>::ypass(), lists[prec][P_Y2].smem >= lists[prec][P_Y4].smem ? P_Y2 : P_Y4))) return rc;
+    if ((rc = attr(PassKernels<T>::template yzpass<256, KS_WT>(), P_YZ))) return rc;
+    if ((rc = attr(PassKernels<T>::template yzpass<512, KS_WT>(), P_YZB))) return rc;
+    if ((rc = attr(PassKernels<T>::template yzpass<256, KS_WGC>(), P_YZG))) return rc;
+    if ((rc = attr(PassKernels<T>::template yzpass<512, KS_WGC>(), P_YZBG))) return rc;
+    if ((rc = attr(PassKernels<T>::template zpass<KS_WT>(), P_Z3))) return rc;
+    return attr(PassKernels<T>::template xinv<KS_WT>(), P_X5);
   }
 
   // Capture `nticks` ticks into one CUDA graph (re-captured when the set of

@@ -1,41 +1,25 @@
-// The pass kernels of the FP32 slots, instantiated by pass_*_f32.cu: the passes
-// without the row split, their twiddles from the plain roots table.  (An FP32
-// solve ends at the precision floor of its line search; there another order
-// of rounding changes which trial it ends on, so the FP32 passes keep theirs.)
-// These headers are a translation unit's whole view of the library: slot.cuh
-// here is the record of ../slot.cuh up to its FP64 plans.
+// The pass kernels of the FP32 slots, as engine.cu sees them (pass_*_f32.cu
+// instantiates them from passes.cuh); in the host emulation, their block
+// functions.
 #pragma once
-#include <cuda_runtime.h>
-
-#include "passes.cuh"
+#include "shape.cuh"
 
 namespace ofdft {
+namespace f32 {
 
-// Minimum resident 256-thread blocks per SM of the x and split y/z passes (it
-// caps the registers at 65536 / (256 * minb)).
-constexpr int PASS_MINB = 4;
-template <typename T, int KS> __global__ void __launch_bounds__(256, PASS_MINB) k_xfwd(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  xfwd_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-template <typename T> __global__ void __launch_bounds__(256, PASS_MINB) k_ypass(Args<T> a, int dir) {
-  extern __shared__ __align__(16) char sm[];
-  ypass_block<T>(a, blockIdx.x, threadIdx.x, blockDim.x, sm, dir);
-}
-template <typename T, int KS> __global__ void __launch_bounds__(256, PASS_MINB) k_zpass(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  zpass_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-// Fused y-z pass: 256-thread blocks, up to three per SM; 512-thread blocks, one
-// per SM, for larger planes.
-template <typename T, int NT, int KS>
-__global__ void __launch_bounds__(NT, NT == 256 ? 3 : 1) k_yzpass(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  yzpass_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
-template <typename T, int KS> __global__ void __launch_bounds__(256, PASS_MINB) k_xinv(Args<T> a) {
-  extern __shared__ __align__(16) char sm[];
-  xinv_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
-}
+#if defined(OFDFT_EMU)
+template <typename T, int KS> void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem);
+template <typename T> void ypass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem, int dir);
+template <typename T, int KS> void zpass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem);
+template <typename T, int KS> void yzpass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem);
+template <typename T, int KS> void xinv_block(const Args<T>& a, int bid, int tid, int nthr, char* smem);
+#else
+template <typename T, int KS> __global__ void k_xfwd(Args<T> a);
+template <typename T> __global__ void k_ypass(Args<T> a, int dir);
+template <typename T, int KS> __global__ void k_zpass(Args<T> a);
+template <typename T, int NT, int KS> __global__ void k_yzpass(Args<T> a);
+template <typename T, int KS> __global__ void k_xinv(Args<T> a);
+#endif
 
+}  // namespace f32
 }  // namespace ofdft

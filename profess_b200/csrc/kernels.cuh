@@ -1,4 +1,4 @@
-// The kernels of the evaluation passes.  They hold most of the library's code
+// The kernels of the FP64 evaluation passes (FP32: f32/kernels.cuh).  They hold most of the library's code
 // (every radix of every stage), so each is instantiated in a translation unit
 // of its own (pass_*.cu): the units compile side by side, and a unit's code
 // does not depend on what else is compiled with it.  engine.cu sees them as
@@ -11,8 +11,6 @@
 
 namespace ofdft {
 
-// The FP32 units (pass_*_f32.cu) take the kernels of f32/kernels.cuh.
-//
 // Minimum resident 256-thread blocks per SM of the kernels (they cap the
 // registers at 65536 / (256 * minb)): the split passes keep three columns of a
 // WGC group in registers (1152 ions, 160 x 160 x 256: z pass 338 us with two
@@ -66,7 +64,6 @@ template <typename T, int KS> __global__ void __launch_bounds__(256, X_MINB) k_x
   OFDFT_SPLIT_KERNELS(T, X)
 
 #if !defined(OFDFT_INSTANTIATE)
-OFDFT_PASS_KERNELS(float, extern)
 OFDFT_PASS_KERNELS(double, extern)
 #endif
 

@@ -1,5 +1,5 @@
-// Block functions of the engine: the vector-op kernel and the passes of one
-// potential evaluation (CalculatePotentialPlus).
+// The FP64 passes of one potential evaluation (CalculatePotentialPlus); the FP32
+// slots' passes are those of f32/passes.cuh.
 //
 // Spectrum layout: field f of a slot is a half spectrum of k1 = n1/2 + 1
 // planes, kx-major: element (kx, row j = y + n2 z) at spec[f*Nc + kx*nrows +
@@ -15,14 +15,14 @@
 //                       forward FFT along y and z, the k-space operator
 //                       (Hartree 4pi/G^2, vW G^2, the WT kernel, with the 1/N
 //                       forward scaling), inverse FFT along z and y
-//   (planes that do not fit shared memory, the WGC groups and the set-up
-//    modes run the same work as three passes: Y forward, Z with the
-//    operator, Y inverse)
+//                       (the three planes of a WGC group together)
+//   (planes that do not fit shared memory and the set-up modes run the same
+//    work as three passes: Y forward, Z with the operator, Y inverse)
 //   pass 5  X inverse : complex-to-real FFT of all fields of a row pair and the
 //                       real-space epilogue (potential, chain rule, energies and
 //                       the optimiser's fused sums)
 //
-// Row split (FP64, n3 even): the x passes do the radix-2 stage of the z transform,
+// Row split (n3 even): the x passes do the radix-2 stage of the z transform,
 // on real values (the sums and differences of rows n3/2 apart), and multiply
 // its twiddles onto the spectra that they hold in registers anyway.  What is
 // left of a plane's z transform is two independent transforms of length n3/2,
@@ -38,33 +38,14 @@
 // that follows (one block per slot) reduces them in a fixed order (the result
 // does not depend on block scheduling) and runs the NTN controller.
 #pragma once
-#include "ntn_ctl.cuh"
+#include "fft.cuh"
+#include "pass_common.cuh"
 
 namespace ofdft {
-
-constexpr double PI_D = 3.141592653589793238462643;
-constexpr double C_TF = 2.87123400018819;  // Source/KEDF_TF.f90:42
-
-// Kernel instantiations per kinetic functional: the WT kernels carry at most
-// 4 fields and no WGC code, so their register allocation is not set by the
-// 8-field WGC paths.
-enum KinSel : int { KS_WT = 0, KS_WGC = 1 };
-template <int KS> struct KinFields { static constexpr int value = KS == KS_WT ? 4 : MAX_FIELDS; };
-
-template <typename T>
-struct Args {
-  SlotDev* slots;
-  Ctl* ctl;
-  const Task* tasks;
-  const cx<T>* tw;   // stage twiddles of every plan (FftPlan::stw)
-  const int* idx;    // digit-reversal tables (FftPlan::perm, iperm)
-  int vchunk;        // points per task of the vector kernel
-};
 
 // Pitch of the x passes' transform buffer: element i of column c at
 // buf[i * pitch + c].  Odd, so that threads walking x (a stride of one pitch)
 // as well as threads walking the columns touch distinct banks.
-HD size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 HD int x_pitch(int cols) { return cols | 1; }
 // Shared memory of an x-forward task with nfb fields (or ion species) and nb
 // columns each.
@@ -76,365 +57,6 @@ HD size_t xinv_smem(int n1, int nfb, int nb, size_t esz) {
   return xinv_buf(n1, nfb, nb, esz) + NCH * 33 * sizeof(double);
 }
 
-// V_loc(|q|) by the index-knot cubic spline (PspRecipCubicSpline, LocalPseudoPot.f90:92-202).
-HD double psp_value(const IonAux& x, int sp, double q) {
-  const PspDev& p = x.psp[sp];
-  if (q == 0.0) return p.v0;
-  if (q >= p.max_g) return 0.0;
-  const double pos = q / p.dq + 1.0;
-  const int left = (int)floor(pos);
-  const double dt = pos - (double)left;
-  const double* vqs = x.tab + p.off;
-  const double* pdd = x.tab + p.off + p.npts;
-  const double yl = vqs[left - 1], yr = vqs[left];
-  const double pl = pdd[left - 1], pr = pdd[left];
-  const double yval = yl + dt * (yr - yl - (pr / 6.0 + pl / 3.0) + dt * (0.5 * pl + dt * ((pr - pl) / 6.0)));
-  return yval - 4.0 * PI_D * p.charge / (q * q);
-}
-
-// ------------------------------------------------------------ reductions
-// Reduce channels [LO, HI) of acc[NCH] over the block; the block totals end
-// up in sred[LO..HI-1] and the other channels of sred[0..NCH-1] are zero.  On
-// the device: warp shuffles, then one warp over the per-warp sums (sred needs
-// NCH * 33 doubles).  In the host emulation the block has one thread.  Passes
-// whose sums use few channels (a CG evaluation one, the vector operations
-// three) reduce only those.
-template <int LO = 0, int HI = NCH>
-HDNI inline void block_reduce(double* sred, const double* acc, int tid, int nthr) {
-#if defined(__CUDA_ARCH__)
-  const int lane = tid & 31, warp = tid >> 5, nw = (nthr + 31) >> 5;
-  double v[NCH];
-#pragma unroll
-  for (int ch = LO; ch < HI; ++ch) {
-    double x = acc[ch];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    v[ch] = x;
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int ch = LO; ch < HI; ++ch) sred[NCH + ch * 32 + warp] = v[ch];
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch) {
-      if (ch < LO || ch >= HI) {
-        if (lane == 0) sred[ch] = 0.0;
-        continue;
-      }
-      double x = lane < nw ? sred[NCH + ch * 32 + lane] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) sred[ch] = x;
-    }
-  }
-  __syncthreads();
-#else
-  (void)tid;
-  (void)nthr;
-  for (int ch = 0; ch < NCH; ++ch) sred[ch] = (ch >= LO && ch < HI) ? acc[ch] : 0.0;
-#endif
-}
-
-// Store this task's per-channel sums (channels [LO, HI), the rest zero) in
-// the slot's partials.
-template <int LO = 0, int HI = NCH>
-HDNI inline void store_partials(SlotDev& s, int task_idx, const double* acc, double* sred, int tid, int nthr) {
-  block_reduce<LO, HI>(sred, acc, tid, nthr);
-  if (tid == 0) {
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch) s.partials[(size_t)task_idx * NCH + ch] = sred[ch];
-  }
-}
-
-// Shared memory of the controller block: the reduction scratch, then a copy
-// of the slot's controller record.
-constexpr size_t CTL_SRED_BYTES = (NCH * 33 + 2) * sizeof(double);
-constexpr size_t CTL_SMEM_BYTES = CTL_SRED_BYTES + sizeof(Ctl);
-static_assert(sizeof(Ctl) % 8 == 0, "the controller record is copied as 8-byte words");
-
-// Copy nbytes (a multiple of 8) as 8-byte words spread over the block.
-HDNI inline void copy_words(void* dst, const void* src, size_t nbytes, int tid, int nthr) {
-  unsigned long long* d = (unsigned long long*)dst;
-  const unsigned long long* s = (const unsigned long long*)src;
-  for (int w = tid; w < (int)(nbytes / 8); w += nthr) d[w] = s[w];
-}
-
-// Controller kernel body, one block per running slot: reduce the partials
-// of the work kernel that just ran (in a fixed order, independent of block
-// scheduling) and advance the slot's NTN state machine.  kid = K_VEC after the
-// vector kernel, K_X5 after pass 5.  The block copies the controller record
-// into shared memory with all its threads; the one thread that runs the
-// state machine reads and writes only the fields it needs there, and the
-// block writes the record back.
-HDNI inline void ctl_block(SlotDev* slots, Ctl* ctls, const Task* tasks, int kid, int bid, int tid, int nthr,
-                           char* smem) {
-  const int si = tasks[bid].slot;
-  SlotDev& s = slots[si];
-  Ctl& c = ctls[si];
-  if (c.status != ST_RUNNING) return;
-  const int what = kid == K_VEC ? c.op : c.ev;
-  if (what == 0) return;
-  double* sred = (double*)smem;
-  Ctl* cs = (Ctl*)(smem + CTL_SRED_BYTES);
-  copy_words(cs, &c, sizeof(Ctl), tid, nthr);
-  const CtlSlot sl = ctl_slot(s);
-  const int nt = s.ntask[kid];
-  double part[NCH];
-#pragma unroll
-  for (int ch = 0; ch < NCH; ++ch) part[ch] = 0.0;
-  for (int t = tid; t < nt; t += nthr) {
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch) part[ch] += s.partials[(size_t)t * NCH + ch];
-  }
-  block_reduce(sred, part, tid, nthr);  // its barriers also publish the copy
-  if (tid == 0) {
-    double red[NCH];
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch) red[ch] = sred[ch];
-    ntn_after(*cs, sl, red, kid, what);
-  }
-  BLOCK_SYNC();
-  copy_words(&c, cs, sizeof(Ctl), tid, nthr);
-}
-
-// ------------------------------------------------------------ vector ops
-// 16-byte packs (4 floats or 2 doubles): the vector operations stream their
-// arrays with one 16-byte load or store per pack and array.
-template <typename T> struct Pack { static constexpr int n = 16 / (int)sizeof(T); };
-template <typename T>
-HD void ld_pack(T* v, const T* p) {
-#if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) {
-    const float4 x = *(const float4*)p;
-    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-  } else {
-    const double2 x = *(const double2*)p;
-    v[0] = x.x; v[1] = x.y;
-  }
-#else
-  for (int l = 0; l < Pack<T>::n; ++l) v[l] = p[l];
-#endif
-}
-template <typename T>
-HD void st_pack(T* p, const T* v) {
-#if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
-  else *(double2*)p = make_double2(v[0], v[1]);
-#else
-  for (int l = 0; l < Pack<T>::n; ++l) p[l] = v[l];
-#endif
-}
-
-// One task of a vector operation over points [i0, i1) of a slot: packs of
-// Pack<T>::n points first (i0 is a multiple of the chunk size, so packs are
-// 16-byte aligned), then the points after the last full pack one at a time.
-template <typename T>
-HD void vec_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
-  const Task t = a.tasks[bid];
-  SlotDev& s = a.slots[t.slot];
-  Ctl& c = a.ctl[t.slot];
-  const int op = c.op;
-  if (c.status != ST_RUNNING || op == OP_NONE) return;
-  T* __restrict__ phi = (T*)s.buf[c.iphi];
-  const T* __restrict__ w0 = (const T*)s.buf[c.iw0];
-  const T* __restrict__ w1 = (const T*)s.buf[c.iw1];
-  T* __restrict__ bb = (T*)s.buf[B_B];
-  T* __restrict__ r = (T*)s.buf[B_R];
-  T* __restrict__ p = (T*)s.buf[B_P];
-  T* __restrict__ d = (T*)s.buf[B_D];
-  const T k = (T)c.opc;
-  const int i0 = t.a * a.vchunk;
-  const int n = (int)s.N;
-  const int i1 = i0 + a.vchunk < n ? i0 + a.vchunk : n;
-  constexpr int VP = Pack<T>::n;
-  const int npk = (i1 - i0) / VP;  // full packs
-  const int it = i0 + npk * VP;    // first point after them
-  double acc[NCH];
-#pragma unroll
-  for (int ch = 0; ch < NCH; ++ch) acc[ch] = 0.0;
-  switch (op) {
-    case OP_SQRT_INIT:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T v[VP];
-        ld_pack(v, phi + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          acc[0] += (double)v[l];
-          v[l] = m_sqrt(v[l] < T(0) ? -v[l] : v[l]);
-        }
-        st_pack(phi + i, v);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        const T rho = phi[i];
-        acc[0] += (double)rho;
-        phi[i] = m_sqrt(rho < T(0) ? -rho : rho);
-      }
-      break;
-    case OP_DLDPHI:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T wv[VP], fv[VP], bv[VP], rv[VP], zv[VP];
-        ld_pack(wv, w0 + i);
-        ld_pack(fv, phi + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          const T v = wv[l] - k * T(2) * fv[l];
-          bv[l] = v;
-          rv[l] = -v;
-          zv[l] = T(0);
-          acc[0] += (double)v * (double)v;
-        }
-        st_pack(bb + i, bv);
-        st_pack(r + i, rv);
-        st_pack(p + i, rv);
-        st_pack(d + i, zv);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        const T v = w0[i] - k * T(2) * phi[i];
-        bb[i] = v;
-        r[i] = -v;
-        p[i] = -v;
-        d[i] = T(0);
-        acc[0] += (double)v * (double)v;
-      }
-      break;
-    case OP_CGSTEP:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T dv[VP], pv[VP], rv[VP], wv[VP], fv[VP];
-        ld_pack(dv, d + i);
-        ld_pack(pv, p + i);
-        ld_pack(rv, r + i);
-        ld_pack(wv, w1 + i);
-        ld_pack(fv, phi + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          const T dn = dv[l] + k * pv[l];
-          const T rn = rv[l] - k * wv[l];
-          dv[l] = dn;
-          rv[l] = rn;
-          const T pd = fv[l] + dn;
-          acc[0] += (double)rn * (double)rn;
-          acc[1] += (double)pd * (double)pd;
-          acc[2] += (double)fv[l] * (double)dn;
-        }
-        st_pack(d + i, dv);
-        st_pack(r + i, rv);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        const T dn = d[i] + k * p[i];
-        const T rn = r[i] - k * w1[i];
-        d[i] = dn;
-        r[i] = rn;
-        const T f = phi[i];
-        const T pd = f + dn;
-        acc[0] += (double)rn * (double)rn;
-        acc[1] += (double)pd * (double)pd;
-        acc[2] += (double)f * (double)dn;
-      }
-      break;
-    case OP_PUPD:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T rv[VP], pv[VP];
-        ld_pack(rv, r + i);
-        ld_pack(pv, p + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          pv[l] = rv[l] + k * pv[l];
-          acc[0] += (double)pv[l] * (double)pv[l];
-        }
-        st_pack(p + i, pv);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        const T pn = r[i] + k * p[i];
-        p[i] = pn;
-        acc[0] += (double)pn * (double)pn;
-      }
-      break;
-    case OP_DIRNEG:
-    case OP_NG1:
-    case OP_SD:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T dv[VP], fv[VP], xv[VP];
-        if (op == OP_DIRNEG) {
-          ld_pack(dv, d + i);
-          ld_pack(xv, p + i);
-        } else if (op == OP_SD) {
-          ld_pack(xv, bb + i);
-        } else {
-          ld_pack(dv, d + i);
-        }
-        ld_pack(fv, phi + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          T dn;
-          if (op == OP_DIRNEG) dn = -(dv[l] - k * xv[l]);
-          else if (op == OP_SD) dn = -xv[l];
-          else dn = dv[l];
-          dv[l] = dn;
-          const T pd = fv[l] + dn;
-          acc[1] += (double)pd * (double)pd;
-          acc[2] += (double)fv[l] * (double)dn;
-        }
-        if (op != OP_NG1) st_pack(d + i, dv);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        T dn;
-        if (op == OP_DIRNEG) dn = -(d[i] - k * p[i]);
-        else if (op == OP_SD) dn = -bb[i];
-        else dn = d[i];
-        if (op != OP_NG1) d[i] = dn;
-        const T f = phi[i];
-        const T pd = f + dn;
-        acc[1] += (double)pd * (double)pd;
-        acc[2] += (double)f * (double)dn;
-      }
-      break;
-    case OP_NG2:
-      for (int q = tid; q < npk; q += nthr) {
-        const int i = i0 + q * VP;
-        T dv[VP], fv[VP], wv[VP];
-        ld_pack(dv, d + i);
-        ld_pack(fv, phi + i);
-        ld_pack(wv, w0 + i);
-#pragma unroll
-        for (int l = 0; l < VP; ++l) {
-          const T dn = dv[l] - fv[l] * k;
-          dv[l] = dn;
-          acc[0] += (double)dn * (double)dn;
-          acc[1] += (double)wv[l] * (double)dn;
-        }
-        st_pack(d + i, dv);
-      }
-      for (int i = it + tid; i < i1; i += nthr) {
-        const T dn = d[i] - phi[i] * k;
-        d[i] = dn;
-        acc[0] += (double)dn * (double)dn;
-        acc[1] += (double)w0[i] * (double)dn;
-      }
-      break;
-    default:
-      break;
-  }
-  store_partials<0, 3>(s, t.a, acc, (double*)smem, tid, nthr);  // vector ops use channels 0-2
-}
-
-// ------------------------------------------------------------ evaluation inputs
-// phi_in = ca * A + cb * B of the current evaluation (or rho itself for the
-// drop-in evaluation), held in registers for a whole block.
-template <typename T>
-struct EvalIn {
-  const T* __restrict__ A;
-  const T* __restrict__ B;
-  T ca, cb;
-  int rho_mode;
-};
-
 // phi_in at a point, in one fixed rounding: the x-forward pass (whose fields
 // the gradient is taken of) and the x-inverse pass (which stores phi_in as the
 // line search's trial) must agree to the last bit, since the finite-difference
@@ -442,42 +64,10 @@ struct EvalIn {
 template <typename T>
 HD T phi_in(T ca, T a, T cb, T b) {
 #if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) return __fmaf_rn(ca, a, __fmul_rn(cb, b));
-  else return __fma_rn(ca, a, __dmul_rn(cb, b));
+  return __fma_rn(ca, a, __dmul_rn(cb, b));
 #else
   return ca * a + cb * b;
 #endif
-}
-
-template <typename T>
-HD EvalIn<T> eval_in(const SlotDev& s, const Ctl& c) {
-  EvalIn<T> e;
-  e.A = (const T*)s.buf[c.iphi];
-  e.B = (const T*)s.buf[c.evb];
-  e.ca = (T)c.ca;
-  e.cb = (T)c.cb;
-  e.rho_mode = (c.ev == EV_RHO || c.ev == EV_STRESS || (c.ev == EV_FORCE && c.force_rho)) ? 1 : 0;
-  return e;
-}
-
-// Functional parameters of the real-space stages, in registers.
-template <typename T>
-struct FieldPar {
-  int wt, pow56, aeqb, sum53;
-  T alpha, beta, rho_s;
-};
-
-template <typename T>
-HD FieldPar<T> field_par(const SlotDev& s) {
-  FieldPar<T> f;
-  f.wt = s.kinetic == KIN_WT;
-  f.pow56 = s.pow56;
-  f.aeqb = s.alpha_eq_beta;
-  f.sum53 = (s.alpha + s.beta - 5.0 / 3.0) < 1e-14 && (s.alpha + s.beta - 5.0 / 3.0) > -1e-14;
-  f.alpha = (T)s.alpha;
-  f.beta = (T)s.beta;
-  f.rho_s = (T)s.rho_s;
-  return f;
 }
 
 // ------------------------------------------------------------ pass 1
@@ -524,12 +114,11 @@ struct RowMap {
 HD RowMap row_map(const SlotDev& s) { return RowMap{s.zs, s.n2 * s.zh, s.n2, s.n2 * s.n3}; }
 
 // A column's pair in the (y, z) planes of the spectra: its first row, whether
-// it has a second one, whether the two may be accessed together, and (column
-// 1) the twiddles W_{n3}^z of its rows' radix-2 z stage.
+// it has a second one, and (column 1) the twiddles W_{n3}^z of its rows' radix-2 z stage.
 template <typename T>
 struct PairIO {
   int row;
-  bool has1, vec, tw;
+  bool has1, tw;
   cx<T> wa, wb;
 };
 template <typename T>
@@ -537,7 +126,6 @@ HD PairIO<T> pair_io(const RowMap& rm, int u, int col, const cx<T>* __restrict__
   PairIO<T> p;
   p.row = rm.row(u, col);
   p.has1 = rm.has1(u);
-  p.vec = p.has1 && ((rm.nrows | p.row) & 1) == 0;
   p.tw = col != 0;
   p.wa = p.wb = mk<T>(T(1), T(0));
   if (p.tw) {
@@ -557,25 +145,15 @@ HD void x_store(cx<T>* __restrict__ o, cx<T> z, cx<T> zn, const PairIO<T>& io) {
     a = cmul(a, io.wa);
     b = cmul(b, io.wb);
   }
-  if (io.vec) {
-    st_cx2(o, a, b);
-  } else {
-    o[0] = a;
-    if (io.has1) o[1] = b;
-  }
+  o[0] = a;
+  if (io.has1) o[1] = b;
 }
 // The loads' mirror: the two rows' values (a, b) of frequency k, and the
 // packed sequence Z = A + i B at k and n - k in their place.
 template <typename T>
 HD void x_load(const cx<T>* __restrict__ o, const PairIO<T>& io, cx<T>& a, cx<T>& b) {
-  if (io.vec) {
-    const Cx2<T> q = ld_cx2(o);
-    a = q.a;
-    b = q.b;
-  } else {
-    a = o[0];
-    b = io.has1 ? o[1] : mk<T>(T(0), T(0));
-  }
+  a = o[0];
+  b = io.has1 ? o[1] : mk<T>(T(0), T(0));
 }
 template <typename T>
 HD void x_untwiddle(cx<T>& a, cx<T>& b, const PairIO<T>& io) {
@@ -664,8 +242,7 @@ HD void x_last_split(const cx<T>* buf, cx<T>* spec, long long Nc, const RowMap& 
 template <typename T>
 HD T add_rn(T a, T b) {
 #if defined(__CUDA_ARCH__)
-  if constexpr (sizeof(T) == 4) return __fadd_rn(a, b);
-  else return __dadd_rn(a, b);
+  return __dadd_rn(a, b);
 #else
   return a + b;
 #endif
@@ -721,16 +298,12 @@ HD void x_gather(cx<T>* __restrict__ buf, const cx<T>* __restrict__ spec, long l
 // rho and sqrt(rho) of an input value (phi_in, or rho itself in rho mode).
 template <typename T> HD T in_rho(T x, int rho_mode) { return rho_mode ? x : x * x; }
 template <typename T> HD T in_sqrt(T x, int rho_mode) { return rho_mode ? m_sqrt(x) : (x < T(0) ? -x : x); }
-// rho^(5/6) of rho and a = sqrt(rho): FP64 a^2 a^(-1/3) (out: a is outside
-// m_icbrt's range), FP32 a cbrt(rho).
+// rho^(5/6) = a^2 a^(-1/3) of rho and a = sqrt(rho) (out: a is outside
+// m_icbrt's range).
 template <typename T>
 HD T pow56(T rho, T a, bool& out) {
-  if constexpr (sizeof(T) == 4) {
-    return a * m_cbrt(rho);
-  } else {
-    out = out || icbrt_out(a);
-    return rho * m_icbrt(a);
-  }
+  out = out || icbrt_out(a);
+  return rho * m_icbrt(a);
 }
 
 // All forward fields of NP points from their evaluation inputs (WT: rho,
@@ -902,32 +475,6 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   x_last_split<T>(buf, (cx<T>*)s.spec, s.Nc, rm, u0, nf, nb, es, px, a.idx + px.iperm, a.tw + s.qz.stw[0], tid, nthr);
 }
 
-// ------------------------------------------------------------ k-space operators
-HD int signed_freq(int k, int n) { return k > n / 2 ? k - n : k; }
-
-// Real factor of the single-field operators at the frequency (m1, m2, m3)
-// (signed): Hartree 4 pi / |G|^2 (0 at G = 0) and vW |G|^2, each times the
-// 1/N forward scale; |G|^2 in the slot's precision.
-template <typename T>
-struct GFactor {
-  T rt[9];
-  T sc, c4;
-  HD void init(const SlotDev& s) {
-#pragma unroll
-    for (int q = 0; q < 9; ++q) rt[q] = (T)s.recip[q];
-    sc = (T)s.inv_n;
-    c4 = (T)(4.0 * PI_D * s.inv_n);
-  }
-  HD T operator()(int kind, int m1, int m2, int m3) const {
-    const T tx = rt[0] * (T)m1 + rt[3] * (T)m2 + rt[6] * (T)m3;
-    const T ty = rt[1] * (T)m1 + rt[4] * (T)m2 + rt[7] * (T)m3;
-    const T tz = rt[2] * (T)m1 + rt[5] * (T)m2 + rt[8] * (T)m3;
-    const T g2 = tx * tx + ty * ty + tz * tz;
-    if (kind == G_VW) return g2 * sc;
-    return (m1 == 0 && m2 == 0 && m3 == 0) ? T(0) : c4 / g2;
-  }
-};
-
 // The operator of one z-pass tile of a set-up mode (G_ION, G_FORCE): res[i*NB
 // + q*nb + b] holds species q at z position z0 + i (frequency kz = permz[z0 +
 // i]) and y position y0 + b (ky = permy[y0 + b]), for kx; the results replace
@@ -976,10 +523,6 @@ HD void zpass_setup(const SlotDev& s, int kind, int gn, cx<T>* res, int NB, int 
     }
   }
 }
-
-// Odd row pitch of a plane or tile held in shared memory with y fastest:
-// transforms along y then take columns at an odd stride (conflict-free).
-HD int odd_pitch(int n) { return n | 1; }
 
 // The last forward stage (radix R, stride 1) of the three columns of a WGC
 // group, the second-order WGC operator (KEDF_WGC.f90:219-236) and the first
@@ -1034,27 +577,7 @@ HD void ip_stage_wgc3(cx<T>* buf, int ncols, unsigned mcols, int cs, int es, int
 #undef OFDFT_RADIX_DO
 }
 
-// Accessors of the fused pass: the plane in global memory (y fastest, row
-// length n2) and in shared memory (rows of odd pitch P); column c is y,
-// position i is z.
-template <typename T>
-struct PlaneIO {
-  cx<T>* p;
-  int pitch;
-  HD cx<T> ld(int y, int z) const { return p[z * pitch + y]; }
-  HD void st(int y, int z, cx<T> v) const { p[z * pitch + y] = v; }
-};
-
-// Operator factors at (column z, y position q) of the fused pass: the WT
-// kernel plane (stored in the transforms' digit-reversed order) times the
-// 1/N forward scale, or the Hartree / vW factor of the frequencies there.
-template <typename T>
-struct KernOp {
-  const T* __restrict__ kern;
-  T sc;
-  int n2;
-  HD T operator()(int z, int q) const { return kern[z * n2 + q] * sc; }
-};
+// The Hartree / vW factor at (column z, y position q) of the fused pass.
 template <typename T>
 struct GOp {
   GFactor<T> gf;
@@ -1230,23 +753,6 @@ HD void zpass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
 }
 
 // ------------------------------------------------------------ YZ pass (fused path)
-// The (y, z) planes at kx of the three fields of a WGC group in the spectra
-// (field p at base + p*Nc), seen as 3*n2 columns c = p*n2 + y of n3
-// positions z.
-template <typename T>
-struct Planes3IO {
-  cx<T>* base;
-  long long Nc;
-  int n2;
-  unsigned mn2;
-  HD size_t at(int c, int z) const {
-    const int p = magic_div32(c, mn2), y = c - p * n2;
-    return (size_t)p * (size_t)Nc + (size_t)z * n2 + y;
-  }
-  HD cx<T> ld(int c, int z) const { return base[at(c, z)]; }
-  HD void st(int c, int z, cx<T> v) const { base[at(c, z)] = v; }
-};
-
 // Task (WGC group g, kx, half): the three fields' (y, z) half planes at kx together in
 // shared memory, interleaved along y (field p, y, z at z*P3 + p*n2 + y, P3 =
 // odd pitch of 3*n2), since the WGC operator mixes the three at each
@@ -1358,9 +864,9 @@ HD void yzpass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
 
 // ------------------------------------------------------------ pass 5
 // Perdew-Zunger LDA potential and energy density (XC_LDA.f90:51-310) from
-// rho, r13 = rho^(1/3), rs = cC / r13 and sr = sqrt(rs) (negative: not known).
+// rho, r13 = rho^(1/3), rs = cC / r13 and sr = sqrt(rs).
 template <typename T>
-HD void lda_point(T rho, T r13, T rs, T sr0, T& vxc, T& exc) {
+HD void lda_point(T rho, T r13, T rs, T sr, T& vxc, T& exc) {
   const T cXp = T(-0.98474502184269641), cXe = T(-0.73855876638202234);
   if (rs < T(1)) {
     const T lr = m_log(rs);
@@ -1368,7 +874,6 @@ HD void lda_point(T rho, T r13, T rs, T sr0, T& vxc, T& exc) {
           T(-8.4e-3) * rs;
     exc = cXe * rho * r13 + rho * (lr * (T(3.11e-2) + T(2e-3) * rs) + T(-4.8e-2) + T(-1.16e-2) * rs);
   } else {
-    const T sr = sr0 < T(0) ? m_sqrt(rs) : sr0;
     const T den = T(1) + T(1.0529) * sr + T(3.334e-1) * rs;
     const T iden = T(1) / den;
     vxc = cXp * r13 + (T(-1.423e-1) + T(-0.174798948333333333) * sr + T(-6.325709333333333333e-2) * rs) *
@@ -1400,7 +905,7 @@ struct XinvEpi {
 // The epilogue of one point: its potential (stored to the mode's output
 // arrays at idx) and its terms of the mode's sums, added to sums[] in the
 // slot precision.  o[f] are the point's field outputs of the inverse
-// transforms; vi its ion potential, phin, rho, sq = sqrt(rho) and (FP64) y =
+// transforms; vi its ion potential, phin, rho, sq = sqrt(rho) and y =
 // rho^(-1/6) its evaluation input, ex and ey its optimiser inputs.
 template <typename T, int EV>
 HD void epi_input(const XinvEpi<T>& e, T aa, T bx, T& phin, T& rho, T& sq) {
@@ -1418,28 +923,21 @@ template <typename T, int KS, int EV, bool ENERGY>
 HD void epi_point(const XinvEpi<T>& e, const T* o, T vi, T phin, T rho, T sq, T y, T ex, T ey, int idx, T* sums) {
   const FieldPar<T> fp = e.fp;
   const T cC = T(0.62035049089940009);
-  T x, r13;  // rho^(-1/3), rho^(1/3)
-  if constexpr (sizeof(T) == 4) {
-    x = m_rcbrt(rho);
-    r13 = rho * x * x;
-  } else {
-    x = y * y;
-    r13 = sq * y;
-  }
+  const T x = y * y, r13 = sq * y;  // rho^(-1/3), rho^(1/3)
   const T r23 = r13 * r13;
   const T rinv = x * x * x;        // 1/rho
   T vxc, exc;
   const T rs = cC * x;
-  lda_point(rho, r13, rs, sizeof(T) == 4 ? T(-1) : T(0.78762331789974329708) * y, vxc, exc);  // sqrt(cC) y
+  lda_point(rho, r13, rs, T(0.78762331789974329708) * y, vxc, exc);  // sqrt(cC) y
   T vnl, enl, lap;
   const T al = e.al, be = e.be, cTF = e.cTF;
   if constexpr (KS == KS_WT) {
     const T pa = e.nf > 3 ? o[3] : o[1];
-    if (sizeof(T) == 8 && fp.pow56) {  // rho^(5/6) = rho y
+    if (fp.pow56) {  // rho^(5/6) = rho y
       vnl = cTF * y * (al * o[1] + be * pa);
       enl = cTF * (rho * y) * o[1];
     } else {
-      const T rbeta = sizeof(T) == 4 && fp.pow56 ? sq * r13 : m_pow(rho, be);
+      const T rbeta = m_pow(rho, be);
       const T ralpha = fp.aeqb ? rbeta : m_pow(rho, al);
       vnl = cTF * (al * (ralpha * rinv) * o[1] + be * (rbeta * rinv) * pa);
       enl = cTF * ralpha * o[1];
@@ -1540,14 +1038,10 @@ HD void xinv_points(const XinvEpi<T>& e, double* acc_out, int tid, int nthr) {
     T p0, p1, rho0, rho1, sq0, sq1;
     epi_input<T, EV>(e, aa0, bx0, p0, rho0, sq0);
     epi_input<T, EV>(e, aa1, bx1, p1, rho1, sq1);
-    T y0 = T(0), y1 = T(0);
-    if constexpr (sizeof(T) == 8) {
-      y0 = m_icbrt(sq0);
-      y1 = m_icbrt(sq1);
-      if (icbrt_out(sq0) || icbrt_out(sq1)) {
-        y0 = m_icbrt_any(sq0);
-        y1 = m_icbrt_any(sq1);
-      }
+    T y0 = m_icbrt(sq0), y1 = m_icbrt(sq1);
+    if (icbrt_out(sq0) || icbrt_out(sq1)) {
+      y0 = m_icbrt_any(sq0);
+      y1 = m_icbrt_any(sq1);
     }
     epi_point<T, KS, EV, ENERGY>(e, o0, vi0, p0, rho0, sq0, y0, ex0, bx0, idx0, sums);
     if (has1) epi_point<T, KS, EV, ENERGY>(e, o1, vi1, p1, rho1, sq1, y1, ex1, bx1, idx1, sums);

@@ -9,7 +9,7 @@
 #pragma once
 #include "cx.cuh"
 #include "dcsrch.cuh"
-#include "fft.cuh"
+#include "dft.cuh"
 
 namespace ofdft {
 
@@ -86,11 +86,10 @@ struct IonAux {
   const cx<double>* b3;   // n3 entries
 };
 
-constexpr int SLOT_BYTES = 2128;
 struct SlotDev {
   int n1, n2, n3, k1;
   long long N, Nc;
-  FftPlan px, py, pz;  // default plans (the FP32 passes)
+  FftPlan px, py, pz;  // default plans (the FP32 passes; their twiddles are the roots)
   double recip[9];  // cellRecip, column-major: recip[3*c + r] = b_c component r
   double dv, inv_n, vol;
   int kinetic, nf, ngroups, alpha_eq_beta;
@@ -108,13 +107,12 @@ struct SlotDev {
   double* partials;  // ntask_max * NCH
   int ntask[NKID];
   HistEntry* hist;
-  // The fields up to here are what the FP32 pass units see (f32/slot.cuh).
+  // FP64:
   StagePlan qx, qxf;   // x-inverse and x-forward pass (the spectra are in natural kx order: the two may differ)
   StagePlan qy, qz;    // y; the whole z axis (the row split's radix first)
   StagePlan qzh;       // the z transforms after the x passes' share (length zh)
   int zs, zh;          // row split: the x passes do the first z stage, of radix zs (1 or 2); zh = n3 / zs
 };
-static_assert(sizeof(SlotDev) == SLOT_BYTES && sizeof(StagePlan) == 212, "the FP32 units' slot record (f32/slot.cuh)");
 
 struct Ctl {
   int status, error, state, op, ev;
