@@ -45,7 +45,7 @@ struct FftPlan {
   int R[FFT_MAX_STAGES];
   int L[FFT_MAX_STAGES];               // block length of stage s, n / (R_0 ... R_{s-1})
   unsigned m_magic[FFT_MAX_STAGES];    // magic32(L[s] / R[s])
-  int root;                            // offset of exp(-2 pi i e / n), e < n, in the twiddle table (FP32 passes)
+  int root;                            // offset of exp(-2 pi i e / n), e < n, in the twiddle table
   int perm;                            // offset of perm (position -> frequency) in the index table
   int iperm;                           // offset of iperm (frequency -> position)
 };

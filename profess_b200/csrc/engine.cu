@@ -276,86 +276,83 @@ static int z_radices(int n, int prec, int rmax, int* rad) {
 // Radix caps the tuner may give an x-axis plan (the first is the default).
 static const int kCaps[2][3] = {{12, 8, 0}, {16, 12, 8}};  // [0] FP64, [1] FP32
 struct PlanTable {
-  std::map<int, StagePlan> plans[2];  // [0] FP64 (OFDFT_FP64), [1] FP32: default radix cap
-  std::map<int, StagePlan> xfwd[2];    // x-forward pass
-  std::map<int, StagePlan> zplan[2];   // whole z axis: the row split's radix, then the default plan of the rest
-  std::map<int, StagePlan> capped[2];  // key cap * 1024 + n: the plans of the other caps
-  void* d_tw64 = nullptr;           // stage twiddles of every plan (FftPlan::stw)
-  void* d_tw32 = nullptr;
+  std::map<int, FftPlan> plans32;      // FP32: key cap * 1024 + n
+  std::map<int, StagePlan> plans64;    // FP64: key cap * 1024 + n
+  std::map<int, StagePlan> xfwd;       // FP64 x-forward pass
+  std::map<int, FftPlan> zplan;        // FP64 whole z axis: the row split's radix, then the default plan of the rest
+  void* d_tw64 = nullptr;           // roots of unity of every length, then the FP64 plans' stage twiddles
+  void* d_tw32 = nullptr;           // the roots
   int* d_idx = nullptr;             // perm and iperm of every plan
 
+  // Every 7-smooth length.  Plans of a length with the same radices share
+  // their tables.
   int build() {
-    std::vector<long double> re, im;  // the twiddle table: stage tables of every plan
-    std::vector<int> idx;
-    for (int n = 1; n <= MAX_N; ++n) {
+    std::vector<cx<double>> t64;
+    std::vector<cx<float>> t32;
+    std::vector<int> idx, lengths, roots;
+    for (int n = 2; n <= MAX_N; ++n) {
       if (!seven_smooth(n)) continue;
-      std::vector<long double> rr(n), ri(n);  // exp(-2 pi i e / n)
-      for (int e = 0; e < n; ++e) {
+      lengths.push_back(n);
+      roots.push_back((int)t64.size());
+      for (int e = 0; e < n; ++e) {  // exp(-2 pi i e / n)
         const long double ang = -2.0L * 3.141592653589793238462643383279502884L * (long double)e / (long double)n;
-        rr[e] = cosl(ang);
-        ri[e] = sinl(ang);
+        const long double re = cosl(ang), im = sinl(ang);
+        t64.push_back(mk<double>((double)re, (double)im));
+        t32.push_back(mk<float>((float)re, (float)im));
       }
-      const int root = (int)re.size();  // the roots themselves, then the plans' stage tables
-      re.insert(re.end(), rr.begin(), rr.end());
-      im.insert(im.end(), ri.begin(), ri.end());
-      if (n & 1) {
-        re.push_back(0.0L);
-        im.push_back(0.0L);
-      }
-      auto add = [&](const int* rad, int nst) {
-        StagePlan p;
-        memset((void*)&p, 0, sizeof(p));
-        p.root = root;
-        std::vector<int> perm(n), iperm(n);
-        fft_plan_fill(p, n, rad, nst, perm.data(), iperm.data());
-        const int end = fft_stage_twiddles(p, (int)re.size(), [&](int off, int j) {
-          if (off >= (int)re.size()) {
-            re.resize(off + 1, 0.0L);
-            im.resize(off + 1, 0.0L);
-          }
-          re[off] = rr[j];
-          im[off] = ri[j];
-        });
-        re.resize(end, 0.0L);
-        im.resize(end, 0.0L);
-        p.perm = (int)idx.size();
-        idx.insert(idx.end(), perm.begin(), perm.end());
-        p.iperm = (int)idx.size();
-        idx.insert(idx.end(), iperm.begin(), iperm.end());
-        return p;
-      };
-      for (int pi = 0; pi < 2; ++pi) {
-        int rad[FFT_MAX_STAGES];
-        for (int ci = 0; ci < 3 && kCaps[pi][ci]; ++ci) {
-          const int nst = fft_radices(n, kCaps[pi][ci], rad);
-          const StagePlan p = add(rad, nst);
-          if (ci == 0) plans[pi][n] = p;
-          else capped[pi][kCaps[pi][ci] * 1024 + n] = p;
+    }
+    if (t64.size() & 1) t64.push_back(mk<double>(0.0, 0.0));
+    struct Made {
+      std::vector<int> rad;
+      StagePlan p;
+      bool staged;
+    };
+    for (size_t l = 0; l < lengths.size(); ++l) {
+      const int n = lengths[l], root = roots[l];
+      std::vector<Made> made;
+      auto add = [&](const int* rad, int nst, bool staged) -> const StagePlan& {
+        const std::vector<int> key(rad, rad + nst);
+        Made* m = nullptr;
+        for (Made& x : made)
+          if (x.rad == key) m = &x;
+        if (!m) {
+          made.push_back(Made{key, StagePlan(), false});
+          m = &made.back();
+          memset((void*)&m->p, 0, sizeof(m->p));
+          m->p.root = root;
+          m->p.perm = (int)idx.size();
+          m->p.iperm = m->p.perm + n;
+          idx.resize(idx.size() + 2 * (size_t)n);
+          fft_plan_fill(m->p, n, rad, nst, idx.data() + m->p.perm, idx.data() + m->p.iperm);
         }
-        xfwd[pi][n] = add(rad, xfwd_radices(n, kCaps[pi][0], rad));
-        zplan[pi][n] = add(rad, z_radices(n, pi, kCaps[pi][0], rad));
-      }
+        if (staged && !m->staged) {
+          const int off = (int)t64.size();
+          t64.resize((size_t)fft_stage_twiddles(m->p, off, [](int, int) {}));
+          fft_stage_twiddles(m->p, off, [&](int o, int j) { t64[o] = t64[root + j]; });
+          m->staged = true;
+        }
+        return m->p;
+      };
+      int rad[FFT_MAX_STAGES];
+      made.reserve(8);
+      for (int ci = 0; ci < 3 && kCaps[0][ci]; ++ci)
+        plans64[kCaps[0][ci] * 1024 + n] = add(rad, fft_radices(n, kCaps[0][ci], rad), true);
+      xfwd[n] = add(rad, xfwd_radices(n, kCaps[0][0], rad), true);
+      zplan[n] = add(rad, z_radices(n, OFDFT_FP64, kCaps[0][0], rad), false);
+      for (int ci = 0; ci < 3 && kCaps[1][ci]; ++ci)
+        plans32[kCaps[1][ci] * 1024 + n] = add(rad, fft_radices(n, kCaps[1][ci], rad), false);
     }
-    const size_t nt = re.size();
-    std::vector<cx<double>> t64(nt);
-    std::vector<cx<float>> t32(nt);
-    for (size_t i = 0; i < nt; ++i) {
-      t64[i] = mk<double>((double)re[i], (double)im[i]);
-      t32[i] = mk<float>((float)re[i], (float)im[i]);
-    }
-    int rc = dmalloc(&d_tw64, nt * sizeof(cx<double>));
-    if (!rc) rc = dmalloc(&d_tw32, nt * sizeof(cx<float>));
+    int rc = dmalloc(&d_tw64, t64.size() * sizeof(cx<double>));
+    if (!rc) rc = dmalloc(&d_tw32, t32.size() * sizeof(cx<float>));
     if (!rc) rc = dmalloc((void**)&d_idx, idx.size() * sizeof(int));
-    if (!rc) rc = h2d(d_tw64, t64.data(), nt * sizeof(cx<double>));
-    if (!rc) rc = h2d(d_tw32, t32.data(), nt * sizeof(cx<float>));
+    if (!rc) rc = h2d(d_tw64, t64.data(), t64.size() * sizeof(cx<double>));
+    if (!rc) rc = h2d(d_tw32, t32.data(), t32.size() * sizeof(cx<float>));
     if (!rc) rc = h2d(d_idx, idx.data(), idx.size() * sizeof(int));
     return rc;
   }
-  // The plan of length n with radix cap cap (0 or the default cap: the default plan).
-  const StagePlan& get(int pi, int n, int cap) const {
-    auto it = capped[pi].find(cap * 1024 + n);
-    return it == capped[pi].end() ? plans[pi].at(n) : it->second;
-  }
+  // The plan of length n with radix cap cap (0: the default).
+  const StagePlan& get64(int n, int cap = 0) const { return plans64.at((cap ? cap : kCaps[0][0]) * 1024 + n); }
+  const FftPlan& get32(int n, int cap = 0) const { return plans32.at((cap ? cap : kCaps[1][0]) * 1024 + n); }
   void release() {
     dfree(d_tw64);
     dfree(d_tw32);
@@ -764,9 +761,12 @@ struct Engine {
 
   // The x plans of a slot (cap 0: the defaults).
   void set_x_plans(SlotDev& s, int pi, int xcap) {
-    s.px = plans.get(pi, s.n1, xcap);
-    s.qx = x_plan(plans.get(pi, s.n1, xcap));
-    s.qxf = plans.xfwd[pi].at(s.n1);
+    if (pi == 0) {
+      s.qx = x_plan(plans.get64(s.n1, xcap));
+      s.qxf = plans.xfwd.at(s.n1);
+    } else {
+      s.px = plans.get32(s.n1, xcap);
+    }
   }
 
   int create_slot(const ofdft_cell_desc* d, int* out) {
@@ -793,12 +793,18 @@ struct Engine {
     s.Nc = (long long)s.k1 * d->n2 * d->n3;
     const int pi = d->precision == OFDFT_FP32 ? 1 : 0;
     set_x_plans(s, pi, 0);
-    s.py = s.qy = plans.plans[pi][d->n2];
     s.zs = z_split(s.n3, h.prec);
     s.zh = s.n3 / s.zs;
-    s.pz = plans.plans[pi][d->n3];
-    s.qz = plans.zplan[pi][d->n3];
-    s.qzh = plans.plans[pi][s.zh];
+    if (pi == 0) {
+      s.qy = plans.get64(s.n2);
+      s.qz = plans.zplan.at(s.n3);
+      s.qzh = plans.get64(s.zh);
+    } else {
+      s.py = plans.get32(s.n2);
+      s.pz = plans.get32(s.n3);
+      static_cast<FftPlan&>(s.qy) = s.py;  // the order of the kernel planes
+      s.qz = s.pz;
+    }
     if (int rc = set_geometry(h, d->lattice)) {
       h.used = false;
       return rc;
@@ -2847,12 +2853,12 @@ static size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Plan of length n (the engine's FP64 radix rule for its use) with its stage
 // twiddles appended to tw at *toff and its digit-reversal tables to idx at
-// *ioff (no heap use).  A plan of a length up to 128 has at most 2 * 128
-// twiddles.
+// *ioff (no heap use).  root: exp(-2 pi i j / n) at root[step * j].  A plan of
+// a length up to 128 has at most 2 * 128 twiddles.
 constexpr int MAX_TW = 2 * MAX_DIM;
 enum PlanUse { FOR_AXIS, FOR_XFWD, FOR_WHOLE_Z };
-static void make_plan(int n, PlanUse use, StagePlan& p, cx<double>* tw, int* toff, int* idx, int* ioff) {
-  memset((void*)&p, 0, sizeof(p));
+static void make_plan(int n, PlanUse use, const cx<double>* root, int step, StagePlan& p, cx<double>* tw, int* toff,
+                      int* idx, int* ioff) {
   int rad[FFT_MAX_STAGES];
   constexpr int rmax = FftMaxRadix<double>::value;
   const int nst = use == FOR_XFWD ? xfwd_radices(n, rmax, rad)
@@ -2860,11 +2866,21 @@ static void make_plan(int n, PlanUse use, StagePlan& p, cx<double>* tw, int* tof
   fft_plan_fill(p, n, rad, nst, idx + *ioff, idx + *ioff + n);
   p.perm = *ioff;
   p.iperm = *ioff + n;
-  *toff = fft_stage_twiddles(p, *toff, [&](int off, int e) {
-    const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)e / (long double)n;
-    tw[off] = mk<double>((double)cosl(a), (double)sinl(a));
-  });
+  if (use == FOR_WHOLE_Z) {  // its roots (of the row split's stage)
+    p.root = *toff;
+    for (int j = 0; j < n; ++j) tw[*toff + j] = root[step * j];
+    *toff += n + (n & 1);
+  } else {
+    *toff = fft_stage_twiddles(p, *toff, [&](int off, int j) { tw[off] = root[step * j]; });
+  }
   *ioff += 2 * n;
+}
+// exp(-2 pi i j / n), j < n.
+static void make_roots(int n, cx<double>* root) {
+  for (int j = 0; j < n; ++j) {
+    const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)j / (long double)n;
+    root[j] = mk<double>((double)cosl(a), (double)sinl(a));
+  }
 }
 }  // namespace noalloc
 #endif
@@ -2900,14 +2916,25 @@ extern "C" int ofdft_calculate_potential_plus_noalloc(const ofdft_cell_desc* d, 
   memset(tw, 0, sizeof(tw));
   int ptab[10 * MAX_DIM];       // their digit-reversal tables
   int twoff = 0, poff = 0;
-  make_plan(d->n1, FOR_AXIS, s.qx, tw, &twoff, ptab, &poff);
+  cx<double> root[3][MAX_DIM];  // of the axes, a length computed once
+  const cx<double>* axis[3];
+  for (int k = 0; k < 3; ++k) {
+    axis[k] = root[k];
+    for (int j = k - 1; j >= 0; --j)
+      if (ns[j] == ns[k]) axis[k] = axis[j];
+    if (axis[k] == root[k]) make_roots(ns[k], root[k]);
+  }
+  make_plan(d->n1, FOR_AXIS, axis[0], 1, s.qx, tw, &twoff, ptab, &poff);
   s.qx = x_plan(s.qx);
-  make_plan(d->n1, FOR_XFWD, s.qxf, tw, &twoff, ptab, &poff);
-  make_plan(d->n2, FOR_AXIS, s.qy, tw, &twoff, ptab, &poff);
+  make_plan(d->n1, FOR_XFWD, axis[0], 1, s.qxf, tw, &twoff, ptab, &poff);
+  make_plan(d->n2, FOR_AXIS, axis[1], 1, s.qy, tw, &twoff, ptab, &poff);
   s.zs = z_split(s.n3, OFDFT_FP64);
   s.zh = s.n3 / s.zs;
-  make_plan(d->n3, FOR_WHOLE_Z, s.qz, tw, &twoff, ptab, &poff);
-  make_plan(s.zh, FOR_AXIS, s.qzh, tw, &twoff, ptab, &poff);
+  StagePlan whole;
+  memset((void*)&whole, 0, sizeof(whole));
+  make_plan(d->n3, FOR_WHOLE_Z, axis[2], 1, whole, tw, &twoff, ptab, &poff);
+  s.qz = whole;
+  make_plan(s.zh, FOR_AXIS, axis[2], s.zs, s.qzh, tw, &twoff, ptab, &poff);
   const double* L = d->lattice;
   auto A = [&](int r, int c) { return L[3 * c + r]; };
   const double det = A(0, 0) * (A(1, 1) * A(2, 2) - A(1, 2) * A(2, 1)) - A(0, 1) * (A(1, 0) * A(2, 2) - A(1, 2) * A(2, 0)) +

@@ -121,24 +121,36 @@ HD void fft_inplace(cx<T>* buf, int ncols, int cs, int es, const StagePlan& p, c
 // Radix sequence of n (7-smooth, n <= 512): the fewest stages with radices
 // up to rmax, then the smallest largest radix; largest radix first.  No heap
 // use (the allocation-free entry point plans with it too).  Returns the
-// number of stages, 0 if n has no such factorisation.
-inline int fft_radices(int n, int rmax, int* out) {
-  static const int kR[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
-  int st[513], big[513], first[513];
-  for (int m = 0; m <= n; ++m) { st[m] = 1 << 20; big[m] = 1 << 20; first[m] = 0; }
-  st[1] = 0;
-  big[1] = 0;
-  for (int m = 2; m <= n; ++m) {
-    if (n % m) continue;
-    for (int R : kR) {
-      if (R > rmax || m % R || st[m / R] >= (1 << 20)) continue;
-      const int cs = st[m / R] + 1, cb = R > big[m / R] ? R : big[m / R];
-      if (cs < st[m] || (cs == st[m] && cb < big[m])) { st[m] = cs; big[m] = cb; first[m] = R; }
+// number of stages, 0 if n has no such factorisation.  One table holds the
+// sequences of every length (a search for each of an engine's 800 plans was a
+// third of its creation).
+constexpr int FFT_MAX_N = 512;
+struct RadixTable {
+  short first[FFT_MAX_RADIX + 1][FFT_MAX_N + 1];  // largest radix of the sequence of m with radices up to rmax (0: none)
+  RadixTable() {
+    static const int kR[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    memset(first, 0, sizeof(first));
+    for (int rmax = 2; rmax <= FFT_MAX_RADIX; ++rmax) {
+      int st[FFT_MAX_N + 1], big[FFT_MAX_N + 1];
+      for (int m = 0; m <= FFT_MAX_N; ++m) st[m] = big[m] = 1 << 20;
+      st[1] = 0;
+      big[1] = 0;
+      for (int m = 2; m <= FFT_MAX_N; ++m)
+        for (int R : kR) {
+          if (R > rmax || m % R || st[m / R] >= (1 << 20)) continue;
+          const int cs = st[m / R] + 1, cb = R > big[m / R] ? R : big[m / R];
+          if (cs < st[m] || (cs == st[m] && cb < big[m])) { st[m] = cs; big[m] = cb; first[rmax][m] = (short)R; }
+        }
     }
   }
-  if (st[n] >= (1 << 20)) return 0;
+};
+inline int fft_radices(int n, int rmax, int* out) {
+  static const RadixTable table;
   int k = 0;
-  for (int m = n; m > 1; m /= first[m]) out[k++] = first[m];
+  for (int m = n; m > 1; m /= table.first[rmax][m]) {
+    if (!table.first[rmax][m]) return 0;
+    out[k++] = table.first[rmax][m];
+  }
   for (int a = 0; a < k; ++a)  // largest first
     for (int b = a + 1; b < k; ++b)
       if (out[b] > out[a]) { const int t = out[a]; out[a] = out[b]; out[b] = t; }

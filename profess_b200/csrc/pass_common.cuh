@@ -21,7 +21,7 @@ struct Args {
   SlotDev* slots;
   Ctl* ctl;
   const Task* tasks;
-  const cx<T>* tw;   // stage twiddles of every plan (FftPlan::stw)
+  const cx<T>* tw;   // roots of unity of every length (FftPlan::root); FP64: and stage twiddles (StagePlan::stw)
   const int* idx;    // digit-reversal tables (FftPlan::perm, iperm)
   int vchunk;        // points per task of the vector kernel
 };

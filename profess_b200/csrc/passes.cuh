@@ -129,8 +129,8 @@ HD PairIO<T> pair_io(const RowMap& rm, int u, int col, const cx<T>* __restrict__
   p.tw = col != 0;
   p.wa = p.wb = mk<T>(T(1), T(0));
   if (p.tw) {
-    p.wa = wz[2 * (2 * u / rm.n2) + 1];
-    p.wb = p.has1 ? wz[2 * ((2 * u + 1) / rm.n2) + 1] : p.wa;
+    p.wa = wz[2 * u / rm.n2];
+    p.wb = p.has1 ? wz[(2 * u + 1) / rm.n2] : p.wa;
   }
   return p;
 }
@@ -472,7 +472,7 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
     ip_stage<T, -1>(buf, nf * nc, mcols, 1, es, px, st, a.tw, tid, nthr);
     BLOCK_SYNC();
   }
-  x_last_split<T>(buf, (cx<T>*)s.spec, s.Nc, rm, u0, nf, nb, es, px, a.idx + px.iperm, a.tw + s.qz.stw[0], tid, nthr);
+  x_last_split<T>(buf, (cx<T>*)s.spec, s.Nc, rm, u0, nf, nb, es, px, a.idx + px.iperm, a.tw + s.qz.root, tid, nthr);
 }
 
 // The operator of one z-pass tile of a set-up mode (G_ION, G_FORCE): res[i*NB
@@ -1077,7 +1077,7 @@ HD void xinv_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   }
   const int es = x_pitch(NB);
   const RowMap rm = row_map(s);
-  x_gather<T>(buf, spec, Nc, rm, u0, nf, nb, es, s.qx, a.idx + s.qx.iperm, a.tw + s.qz.stw[0], tid, nthr);
+  x_gather<T>(buf, spec, Nc, rm, u0, nf, nb, es, s.qx, a.idx + s.qx.iperm, a.tw + s.qz.root, tid, nthr);
   BLOCK_SYNC();
   {
     const unsigned mcols = magic32(NB);

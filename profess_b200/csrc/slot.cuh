@@ -109,7 +109,8 @@ struct SlotDev {
   HistEntry* hist;
   // FP64:
   StagePlan qx, qxf;   // x-inverse and x-forward pass (the spectra are in natural kx order: the two may differ)
-  StagePlan qy, qz;    // y; the whole z axis (the row split's radix first)
+  StagePlan qy;
+  FftPlan qz;          // the whole z axis, the row split's radix first (its order and roots)
   StagePlan qzh;       // the z transforms after the x passes' share (length zh)
   int zs, zh;          // row split: the x passes do the first z stage, of radix zs (1 or 2); zh = n3 / zs
 };
