@@ -74,31 +74,45 @@ HD float m_rcbrt(float v) { return 1.0f / cbrtf(v); }
 HD double m_rsqrt(double v) { return 1.0 / sqrt(v); }
 #endif
 
-// a^(-1/3) of a in [1e-30, 1e30] (icbrt_out says when it is not: the caller
-// then takes m_icbrt_any, once for a whole group of values, so that the fast
-// path is free of branches).  A single-precision seed y (exp2 of -log2(a)/3 of
-// the float with a's leading bits; relative error about 1e-6) and one step of
-// the series of (1 - e)^(-1/3), e = 1 - a y^3: y (1 + e/3 + 2 e^2/9) (the next
-// term is below 1e-17).  Largest relative error over [1e-5, 10] 1.5e-16
-// (rcbrt: 1.1e-16); with the seed by conversions 47 cycles a warp against 71,
-// by bits fewer.
+// a^(-1/3) and, in m_icbrt2, a^(-2/3) of a in [1e-30, 1e30] (icbrt_out says when
+// it is not: the caller then takes m_icbrt_any, once for a whole group of
+// values, so that the fast path is free of branches).  A single-precision seed
+// y (exp2 of -log2(a)/3 of the float with a's leading bits) and one step of the
+// series of (1 - e)^(-1/3) and (1 - e)^(-2/3) in e = 1 - a y^3 on y and y^2, which
+// is exact: a seed has 24 bits.  The seed's error is about 1e-6 near a = 1 and
+// grows with |log2 a| to 3e-6 at the ends of the range; the first term left out,
+// 35/243 e^4 and 110/243 e^4, is below 1e-20.  What remains is the rounding of a y in
+// e and of the result, as in rcbrt.  rho^(-1/3) as the square of rho^(-1/6) has twice that
+// error, and its cube, 1/rho, six times (RMS error of rho^(-1/3) over [1e-5, 10]
+// 1.1e-16 that way, 5e-17 by the second series and by rcbrt).
 HD bool icbrt_out(double a) { return !(a >= 1e-30 && a <= 1e30); }
 #if defined(__CUDA_ARCH__)
-__device__ __forceinline__ float icbrt_seed(float a) {
-  float s = -0.333333343f * __log2f(a);
+__device__ __forceinline__ double icbrt_seed(double a) {
+  const int h = ((__double2hiint(a) - 0x38000000) << 3) | (int)((unsigned)__double2loint(a) >> 29);
+  float s = -0.333333343f * __log2f(__int_as_float(h));
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(s));
-  return s;
+  const int b = __float_as_int(s);
+  return __hiloint2double((b >> 3) + 0x38000000, b << 29);
 }
 #endif
 HD double m_icbrt(double a) {
 #if defined(__CUDA_ARCH__)
-  const int h = ((__double2hiint(a) - 0x38000000) << 3) | (int)((unsigned)__double2loint(a) >> 29);
-  const int b = __float_as_int(icbrt_seed(__int_as_float(h)));
-  const double y = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+  const double y = icbrt_seed(a);
   const double e = fma(-(a * y), y * y, 1.0);
-  return fma(y * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y);
+  return fma(y * e, fma(e, fma(e, 14.0 / 81.0, 2.0 / 9.0), 1.0 / 3.0), y);
 #else
   return 1.0 / cbrt(a);
+#endif
+}
+HD void m_icbrt2(double a, double& y1, double& y2) {
+#if defined(__CUDA_ARCH__)
+  const double y = icbrt_seed(a), s = y * y;
+  const double e = fma(-(a * y), s, 1.0);
+  y1 = fma(y * e, fma(e, fma(e, 14.0 / 81.0, 2.0 / 9.0), 1.0 / 3.0), y);
+  y2 = fma(s * e, fma(e, fma(e, 40.0 / 81.0, 5.0 / 9.0), 2.0 / 3.0), s);
+#else
+  y1 = 1.0 / cbrt(a);
+  y2 = 1.0 / cbrt(a * a);
 #endif
 }
 #if defined(__CUDA_ARCH__)

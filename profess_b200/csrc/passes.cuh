@@ -905,8 +905,8 @@ struct XinvEpi {
 // The epilogue of one point: its potential (stored to the mode's output
 // arrays at idx) and its terms of the mode's sums, added to sums[] in the
 // slot precision.  o[f] are the point's field outputs of the inverse
-// transforms; vi its ion potential, phin, rho, sq = sqrt(rho) and y =
-// rho^(-1/6) its evaluation input, ex and ey its optimiser inputs.
+// transforms; vi its ion potential, phin, rho, sq = sqrt(rho), y = rho^(-1/6)
+// and x = rho^(-1/3) its evaluation input, ex and ey its optimiser inputs.
 template <typename T, int EV>
 HD void epi_input(const XinvEpi<T>& e, T aa, T bx, T& phin, T& rho, T& sq) {
   if (EV == EV_RHO) {  // the input is rho itself
@@ -920,10 +920,11 @@ HD void epi_input(const XinvEpi<T>& e, T aa, T bx, T& phin, T& rho, T& sq) {
   }
 }
 template <typename T, int KS, int EV, bool ENERGY>
-HD void epi_point(const XinvEpi<T>& e, const T* o, T vi, T phin, T rho, T sq, T y, T ex, T ey, int idx, T* sums) {
+HD void epi_point(const XinvEpi<T>& e, const T* o, T vi, T phin, T rho, T sq, T y, T x, T ex, T ey, int idx,
+                  T* sums) {
   const FieldPar<T> fp = e.fp;
   const T cC = T(0.62035049089940009);
-  const T x = y * y, r13 = sq * y;  // rho^(-1/3), rho^(1/3)
+  const T r13 = sq * y;            // rho^(1/3)
   const T r23 = r13 * r13;
   const T rinv = x * x * x;        // 1/rho
   T vxc, exc;
@@ -1038,13 +1039,17 @@ HD void xinv_points(const XinvEpi<T>& e, double* acc_out, int tid, int nthr) {
     T p0, p1, rho0, rho1, sq0, sq1;
     epi_input<T, EV>(e, aa0, bx0, p0, rho0, sq0);
     epi_input<T, EV>(e, aa1, bx1, p1, rho1, sq1);
-    T y0 = m_icbrt(sq0), y1 = m_icbrt(sq1);
+    T y0, y1, x0, x1;
+    m_icbrt2(sq0, y0, x0);
+    m_icbrt2(sq1, y1, x1);
     if (icbrt_out(sq0) || icbrt_out(sq1)) {
       y0 = m_icbrt_any(sq0);
       y1 = m_icbrt_any(sq1);
+      x0 = m_icbrt_any(rho0);
+      x1 = m_icbrt_any(rho1);
     }
-    epi_point<T, KS, EV, ENERGY>(e, o0, vi0, p0, rho0, sq0, y0, ex0, bx0, idx0, sums);
-    if (has1) epi_point<T, KS, EV, ENERGY>(e, o1, vi1, p1, rho1, sq1, y1, ex1, bx1, idx1, sums);
+    epi_point<T, KS, EV, ENERGY>(e, o0, vi0, p0, rho0, sq0, y0, x0, ex0, bx0, idx0, sums);
+    if (has1) epi_point<T, KS, EV, ENERGY>(e, o1, vi1, p1, rho1, sq1, y1, x1, ex1, bx1, idx1, sums);
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch) acc[ch] += (double)sums[ch];
   }
