@@ -307,14 +307,14 @@ HD T pow56(T rho, T a, bool& out) {
 }
 
 // All forward fields of NP points from their evaluation inputs (WT: rho,
-// rho^beta, sqrt(rho) and, when alpha != beta, rho^alpha; WGC: rho, sqrt(rho),
+// rho^beta, sqrt(rho) - shift and, when alpha != beta, rho^alpha; WGC: rho, sqrt(rho) - shift,
 // then for x = alpha and x = beta: rho^x, theta rho^x, theta^2 rho^x / 2 with
 // theta = rho - rho*), with each power computed once per point: put(f, v) for
 // every field.  POW56: the WT functional with both exponents 5/6 (its fall-back
 // power is a call).  Every index is a constant: arrays indexed in a loop go to
 // local memory.
 template <typename T, int KS, bool POW56, int NP, class Put>
-HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Put put) {
+HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, T shift, const T* x, Put put) {
   T rho[NP], sq[NP], v[NP];
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
@@ -322,7 +322,9 @@ HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Pu
     sq[k] = in_sqrt(x[k], rho_mode);
   }
   put(0, rho);
-  put(KS == KS_WT ? 2 : 1, sq);
+#pragma unroll
+  for (int k = 0; k < NP; ++k) v[k] = sq[k] - shift;
+  put(KS == KS_WT ? 2 : 1, v);
   if constexpr (KS == KS_WT) {
     if constexpr (POW56) {
       bool slow = false;
@@ -360,6 +362,34 @@ HD void point_fields(const FieldPar<T>& fp, int rho_mode, int nf, const T* x, Pu
   }
 }
 
+// The constant that sqrt(rho) is transformed without: the mean of sqrt(rho) at
+// 32 points spread over the cell (a lane's share each; every warp has the same
+// sum).  The von Weizsaecker term takes the Laplacian of sqrt(rho), which a
+// constant is not in, and multiplies the transform's rounding errors, which
+// are of the size of what is transformed, by up to the largest |G|^2: they
+// are most of the error of a potential (RMS over the potential's, 96^3: 2.7e-14
+// with sqrt(rho) whole, 1.0e-14 so; 3 us of 230 of the pass for 16 cells, 26 with
+// eight points that every thread reads).
+template <typename T>
+HD T vw_shift(const EvalIn<T>& in, const SlotDev& s, int tid) {
+  auto at = [&](int k) {
+    const int i = (((k * s.n3) >> 5) * s.n2 + (((k * 7 & 31) * s.n2) >> 5)) * s.n1 + (((k * 11 & 31) * s.n1) >> 5);
+    T x = in.A[i];
+    if (!in.rho_mode) x = in.cb != T(0) ? in.ca * x + in.cb * in.B[i] : in.ca * x;
+    return in_sqrt(x, in.rho_mode);
+  };
+#if defined(__CUDA_ARCH__)
+  T sum = at(tid & 31);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#else
+  (void)tid;
+  T sum = T(0);
+  for (int k = 0; k < 32; ++k) sum += at(k);
+#endif
+  return sum * T(1.0 / 32.0);
+}
+
 template <int N> struct Count { static constexpr int value = N; };
 
 // Every field of a range of units in one block: element i of column f*nc +
@@ -381,6 +411,7 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   cx<T>* buf = (cx<T>*)smem;
   const EvalIn<T> in = eval_in<T>(s, c);
   const FieldPar<T> fp = field_par<T>(s);
+  const T shift = setup ? T(0) : vw_shift(in, s, tid);
   const unsigned mn1 = magic32(n1);
   const bool two = !in.rho_mode && in.cb != T(0);
   // the inputs of NP points at once: every load of both arrays first.  A
@@ -423,13 +454,13 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
         const int idx[1] = {i0};
         T x[1];
         inputs(Count<1>(), in.A, idx, x);
-        point_fields<T, KS, false, 1>(fp, in.rho_mode, nf, x,
+        point_fields<T, KS, false, 1>(fp, in.rho_mode, nf, shift, x,
                                       [&](int f, const T* v) { d[2 * (f * nc)] = has ? v[0] : T(0); });
       } else {
         const int idx[2] = {i0, i0 + rm.half * n1};
         T x[2];
         inputs(Count<2>(), in.A, idx, x);
-        point_fields<T, KS, false, 2>(fp, in.rho_mode, nf, x, [&](int f, const T* v) {
+        point_fields<T, KS, false, 2>(fp, in.rho_mode, nf, shift, x, [&](int f, const T* v) {
           d[2 * (f * nc)] = has ? add_rn(v[0], v[1]) : T(0);
           d[2 * (f * nc + nb)] = has ? add_rn(v[0], -v[1]) : T(0);
         });
@@ -450,7 +481,7 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
           inputs(Count<2>(), A, idx, x);
           auto put = [&](int f, const T* v) { d[f * nc] = mk<T>(v[0], has1 ? v[1] : T(0)); };
           if (setup) put(f0, x);
-          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 2>(fp, in.rho_mode, nf, x, put);
+          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 2>(fp, in.rho_mode, nf, shift, x, put);
         } else {
           const int hs = rm.half * n1;
           const int idx[4] = {i0, i1, i0 + hs, i1 + hs};
@@ -461,7 +492,7 @@ HD void xfwd_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
             d[f * nc + nb] = mk<T>(add_rn(v[0], -v[2]), has1 ? add_rn(v[1], -v[3]) : T(0));
           };
           if (setup) put(f0, x);
-          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 4>(fp, in.rho_mode, nf, x, put);
+          else if constexpr (KS == KS_WT) point_fields<T, KS, true, 4>(fp, in.rho_mode, nf, shift, x, put);
         }
       }
     }
