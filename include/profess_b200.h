@@ -150,9 +150,12 @@ int ofdft_slot_forces(ofdft_engine* e, int slot, const double* rho, int include_
  * size of the fused y-z pass - and keeps the fastest.  The choice is cached
  * in the engine for that kind and applied to every such slot, also to those
  * created later.  ms_default / ms_tuned: the median batched evaluation time
- * before and after; shape[4] (may be NULL): radix cap, x-forward and
- * x-inverse row pairs, y-z threads (0: split y/z path).  No slot may be
- * running; the timed slots' solve records are overwritten. */
+ * before and after; shape[4] (may be NULL): radix cap (FP64 slots: of the
+ * x-inverse pass; the x-forward pass has plans of its own), x-forward (FP64: at
+ * most; each launch takes the task size that suits its cells) and x-inverse row
+ * pairs, y-z threads (0: split y/z path, or an FP64 slot whose launches take
+ * 64 to 256 threads by what they hold).  No slot may be running; the timed
+ * slots' solve records are overwritten. */
 int ofdft_engine_tune(ofdft_engine* e, int slot, int iters, double* ms_default, double* ms_tuned, int* shape);
 /* Pin the slot's launch shape (the four values ofdft_engine_tune reports, e.g.
  * a shape tuned in an earlier run; radix cap 0 and y-z threads 0 mean the

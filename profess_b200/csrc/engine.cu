@@ -1784,9 +1784,11 @@ struct Engine {
   // (passes 1-5 and the controller kernel), timed with events on the engine stream.
   // ---------------------------------------------------------- autotuning
   // The launch shape a tuner may change, per slot: the radix cap of the x-axis
-  // FFT plan, row pairs per x-forward and per x-inverse task, and the block
-  // size of the fused y-z pass (256 or 512 threads; 0 = by plane size).  The
-  // y and z plans stay fixed: the kernel planes are stored in their order.
+  // FFT plan (FP64: of the x-inverse pass's), row pairs per x-forward (FP64: at
+  // most, see xfwd_points) and per x-inverse task, and the block size of the
+  // fused y-z pass (256 or 512 threads; 0 = by plane size, FP64 planes of the
+  // small class by launch).  The y and z plans stay fixed: the kernel planes
+  // are stored in their order.
   struct Shape {
     int xcap, rp1, rp, yzt;
   };
@@ -1969,7 +1971,9 @@ struct Engine {
     v[0] = h.xcap ? h.xcap : kCaps[pi][0];
     v[1] = h.rp1;
     v[2] = h.sd.rp;
-    v[3] = uses_yz(h) ? (h.yzt ? h.yzt : (yz_smem_slot(h.sd, csz) <= YZ_SMEM_SMALL ? 256 : 512)) : 0;
+    // not pinned: 0 where each launch takes its own number (yz_threads)
+    const bool small = yz_smem_slot(h.sd, csz) <= YZ_SMEM_SMALL;
+    v[3] = !uses_yz(h) ? 0 : h.yzt ? h.yzt : !small ? 512 : h.prec == OFDFT_FP32 ? 256 : 0;
     return OFDFT_OK;
   }
 
