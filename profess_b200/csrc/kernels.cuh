@@ -12,19 +12,22 @@
 namespace ofdft {
 
 // Minimum resident 256-thread blocks per SM of the kernels (they cap the
-// registers at 65536 / (256 * minb)): the split passes keep three columns of a
-// WGC group in registers (1152 ions, 160 x 160 x 256: z pass 338 us with two
-// blocks, 387 with three).
-constexpr int SPLIT_MINB = 2, X_MINB = 3, YZ_MINB = 3;
+// registers at 65536 / (256 * minb)): three, but for the z pass of a WGC cell,
+// which keeps three columns in registers (160 x 160 x 256: 336 us with two
+// blocks, 384 with three; 100 x 100 x 128: 98 and 112; WT z pass: 180^3 136 and 119,
+// 512 x 128 x 256 383 and 325; y pass: 100 x 100 x 128 WGC 53 and 44, 512 x 128 x
+// 256 249 and 223, 180^3 103 and 104).
+constexpr int X_MINB = 3, Y_MINB = 3, YZ_MINB = 3;
+constexpr int z_minb(int ks) { return ks == KS_WGC ? 2 : 3; }
 template <typename T, int KS> __global__ void __launch_bounds__(256, X_MINB) k_xfwd(Args<T> a) {
   extern __shared__ __align__(16) char sm[];
   xfwd_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
 }
-template <typename T> __global__ void __launch_bounds__(256, SPLIT_MINB) k_ypass(Args<T> a, int dir) {
+template <typename T> __global__ void __launch_bounds__(256, Y_MINB) k_ypass(Args<T> a, int dir) {
   extern __shared__ __align__(16) char sm[];
   ypass_block<T>(a, blockIdx.x, threadIdx.x, blockDim.x, sm, dir);
 }
-template <typename T, int KS> __global__ void __launch_bounds__(256, SPLIT_MINB) k_zpass(Args<T> a) {
+template <typename T, int KS> __global__ void __launch_bounds__(256, z_minb(KS)) k_zpass(Args<T> a) {
   extern __shared__ __align__(16) char sm[];
   zpass_block<T, KS>(a, blockIdx.x, threadIdx.x, blockDim.x, sm);
 }
