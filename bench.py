@@ -74,11 +74,12 @@ def _peaks():
 
 
 def source_sha() -> str:
-    """SHA-256 (first 16 hex digits) of the engine's CUDA sources: the build a
-    profile describes."""
+    """SHA-256 (first 16 hex digits) of the engine's CUDA sources, those in
+    folders below csrc among them: the build a profile describes."""
     h = hashlib.sha256()
     csrc = os.path.join(ROOT, "profess_b200", "csrc")
-    for name in sorted(os.listdir(csrc)):
+    names = [os.path.relpath(os.path.join(d, f), csrc) for d, _, files in os.walk(csrc) for f in files]
+    for name in sorted(names):
         if name.endswith((".cu", ".cuh")):
             with open(os.path.join(csrc, name), "rb") as fh:
                 h.update(name.encode() + b"\0" + fh.read())
