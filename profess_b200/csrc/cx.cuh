@@ -51,7 +51,6 @@ template <typename T> HD cx<T> mul_i(cx<T> a, int dir) {
 // Precision-generic math wrappers (float versions map to the float library calls).
 HD double m_sqrt(double v) { return sqrt(v); }
 HD float m_sqrt(float v) { return sqrtf(v); }
-HD double m_cbrt(double v) { return cbrt(v); }
 HD float m_cbrt(float v) { return cbrtf(v); }
 HD double m_pow(double a, double b) { return pow(a, b); }
 HD float m_pow(float a, float b) { return powf(a, b); }
@@ -65,11 +64,9 @@ HD double m_pow_call(double a, double b) { return pow(a, b); }
 HD double m_log(double v) { return log(v); }
 HD float m_log(float v) { return logf(v); }
 #if defined(__CUDA_ARCH__)
-HD double m_rcbrt(double v) { return rcbrt(v); }
 HD float m_rcbrt(float v) { return rcbrtf(v); }
 HD double m_rsqrt(double v) { return rsqrt(v); }
 #else
-HD double m_rcbrt(double v) { return 1.0 / cbrt(v); }
 HD float m_rcbrt(float v) { return 1.0f / cbrtf(v); }
 HD double m_rsqrt(double v) { return 1.0 / sqrt(v); }
 #endif

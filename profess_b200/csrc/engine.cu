@@ -115,10 +115,10 @@ static double xfwd_cost(long long tasks, double points, size_t smem, int sms) {
 // depend on what else is launched, as the x-forward pass's does.  With the row
 // split 66 KB and 24 row pairs, more where a cell has work for 148 tasks of
 // more (every task is a fixed chain of latencies; but larger tasks than that
-// leave the spilled registers no L1: 16 x 96^3 354 us with 12, 368 with 14; 3 x
-// 72^3 30 us with 18, 42 with 14); without it 72 KB and 32 (12 x 45^3: 29 us, 41
-// with 24; 6 x 75^3: 71 us with 20, 79 with 15); WGC 68 KB (4 x 64^3 80 us with
-// 8, 91 with 6).
+// leave the spilled registers no L1: 16 x 96^3 333 us with 12, 342 with 14; 3 x
+// 72^3 28 us with 18, 40 with 16); without it 72 KB and 32 (12 x 45^3: 27 us, 39
+// with 24; 6 x 75^3: 72 us with 19, 77 with 16); WGC 68 KB (4 x 64^3 77 us with
+// 8, 89 with 6).
 static int xinv_row_pairs(const SlotDev& s) {
   const int nrp = (s.n2 * s.n3 + 1) / 2;
   const size_t kb = s.kinetic == KIN_WGC ? 68 : s.zs == 1 ? 72 : 66;
@@ -129,8 +129,8 @@ static int xinv_row_pairs(const SlotDev& s) {
 
 // An x-forward launch's cells.  The task size changes no result (each column is
 // transformed by itself), so a launch takes the points a task whose model time
-// for all its cells is least.  16 x 96^3 FP64: 258 us with 12 row pairs for every
-// batch, 227 with the 16 of this rule; 8 x 64^3 52 -> 38; one 108^3 40 -> 24.
+// for all its cells is least.  16 x 96^3 FP64: 265 us with 12 row pairs for every
+// batch, 232 with the 16 of this rule; 8 x 64^3 52 -> 40; one 108^3 40 -> 25.
 struct XfwdCell {
   int n1, zs, nunits, nf, rp_max;
   // units of a task of about that many points
@@ -199,10 +199,11 @@ static size_t yz_smem_slot(const SlotDev& s, size_t csz) {
   return s.kinetic == KIN_WGC ? (size_t)s.zh * ((3 * s.n2) | 1) * csz : yz_smem(s, csz);
 }
 constexpr size_t YZ_SMEM_MAX = 226 * 1024;
-// Planes up to this size run 256-thread blocks (three per SM up to 75 KB, two
-// up to 112 KB), larger ones one 512-thread block per SM.  Two 256-thread
-// blocks beat one 512-thread block on 84-99 KB plane sets (WT 72^3 FP64,
-// 108^3 FP32, WGC 64^3 FP32: 9-11 % faster evaluations).
+// Planes up to this size (FP64: half planes) run blocks of up to 256 threads
+// (three of 256 per SM up to 75 KB, two up to 112 KB), larger ones one
+// 512-thread block per SM.  Two 256-thread blocks beat one 512-thread block on
+// 84-99 KB (one 108^3 FP32, 64^3 WGC FP32: 9-11 % faster evaluations; FP64 6 x 75^3
+// 106 us of the pass and 116, one 108^3 54 and 61).
 constexpr size_t YZ_SMEM_SMALL = 112 * 1024;
 // Threads of the blocks of an FP64 launch of the small class.  They change no
 // result, so a launch takes the number whose model time is least: whole waves

@@ -691,7 +691,7 @@ struct TileG {  // the Hartree or vW factor there
 // inverse stage run in registers, and the last inverse stage stores straight
 // to the spectra: half of the round trips through shared memory of a staged
 // tile, generic stages and a separate operator loop (1152 ions, 160 x 160 x
-// 256 WGC: FP64 832 -> 338 us, FP32 602 -> 204 us).
+// 256 WGC: 832 -> 338 us).
 template <typename T, int KS>
 HD void zpass_block(const Args<T>& a, int bid, int tid, int nthr, char* smem) {
   const Task t = a.tasks[bid];
