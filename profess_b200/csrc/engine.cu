@@ -291,6 +291,11 @@ struct PlanTable {
     std::vector<cx<double>> t64;
     std::vector<cx<float>> t32;
     std::vector<int> idx, lengths, roots;
+    // Room for every table: the vector does not move while it grows.  Once a
+    // block of 4 MB has been freed, glibc also keeps up to twice that mapped
+    // instead of returning it: with 2 MB the results of 16 cells of 32^3 were
+    // faulted in again for every batch (2.6 ms of result calls for 0.95).
+    t64.reserve(size_t(1) << 18);
     for (int n = 2; n <= MAX_N; ++n) {
       if (!seven_smooth(n)) continue;
       lengths.push_back(n);
